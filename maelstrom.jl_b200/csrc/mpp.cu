@@ -21,7 +21,7 @@
 #include "mpp_fgmres.cuh"
 #include "mpp_levelset.cuh"
 #include "mpp_tma.cuh"
-#include "mpp_cmg.cuh"
+#include "mpp_cluster.cuh"
 #include "mpp_group.cuh"
 
 using namespace mpp;
@@ -149,10 +149,13 @@ struct mpp_ctx {
     BotArgs bot;
     size_t bot_smem, restrict_smem;
     void* botb;  // level lb's right-hand side (natural order, stencil precision)
-    // levels cmg_ls .. lb-1 resident in one cluster of cmg_cs CTAs (k_cmg), when cmg_ls > 0
+    // levels cmg_ls .. L-1 resident in one cluster of cmg_cs CTAs (k_cluster), when cmg_ls > 0
     int cmg_ls, cmg_cs;
     size_t cmg_smem;
-    CmgSlab cmg_slab[CMG_MAXLEV];
+    ClLev cmg_lev[CL_MAXLEV + 1];
+    int cmg_nd, cmg_nact;  // levels spread over the cluster, CTAs that hold planes of them
+    ClLists cmg_l;
+    unsigned cmg_orb, cmg_ogi;
     // TMA tensor maps of the row-split levels the smoother streams with cp.async.bulk.tensor
     TmaLev tma[MAXLEV];
     bool tma_ok[MAXLEV];
@@ -230,6 +233,25 @@ Lev<M> view(const mpp_ctx* c, int l) {
     return v;
 }
 
+// k_cluster's arguments: levels cmg_ls .. L-1.
+template <class M>
+ClArgs<M> cluster_args(const mpp_ctx* c, int sweeps) {
+    ClArgs<M> a;
+    memset(&a, 0, sizeof(a));
+    a.nl = c->L - 1 - c->cmg_ls;
+    a.nd = c->cmg_nd;
+    a.nact = c->cmg_nact;
+    a.sweeps = sweeps;
+    a.coarse = c->opts.coarse;
+    a.l = c->cmg_l;
+    a.orb = c->cmg_orb;
+    a.ogi = c->cmg_ogi;
+    a.fault = &c->sc->s.fault;
+    a.cl = c->bot.lv[c->bot.nl - 1];
+    for (int q = 0; q <= a.nl; q++) a.s[q] = c->cmg_lev[q];
+    for (int q = 0; q < a.nl; q++) a.g[q] = view<M>(c, c->cmg_ls + q);
+    return a;
+}
 int grid_cells(const mpp_ctx* c, int64_t n) {
     int64_t g = (n + TPB - 1) / TPB;
     int64_t cap = (int64_t)c->nsm * MAXBLOCKS_PER_SM;
@@ -270,7 +292,7 @@ void launch_serial(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cu
     cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// A launch of one thread-block cluster of `cs` CTAs (k_cmg), with programmatic dependent
+// A launch of one thread-block cluster of `cs` CTAs (k_cluster), with programmatic dependent
 // launch like the others.
 template <typename... KArgs, typename... Args>
 void launch_cluster(void (*kern)(KArgs...), int cs, int block, size_t smem, cudaStream_t st, Args... args) {
@@ -350,17 +372,13 @@ void prof_size(const mpp_ctx* c, int fam, int level, double& bytes, int64_t& cel
         case F_TRUE: cells = act(level); bpc = 1 + 2 * v + p; break;
         case F_GRADIENT: cells = N; bpc = 1 + 4 + 4 + 24 + 3; break;
         case F_CONVERT: cells = N; bpc = 12; break;
-        case F_CMG: {  // levels cmg_ls .. lb-1 in shared memory: what crosses to global memory
+        case F_CMG: {  // levels cmg_ls .. L-1 in shared memory: what crosses to global memory
+            // codes and diagonals of every level in, b of level ls in, its x out
             cells = 0;
             double b = 0;
-            for (int l = c->cmg_ls; l < c->lb; l++) {
-                const double n = (double)lcells(l);
+            for (int l = c->cmg_ls; l < c->L; l++) {
                 cells += lcells(l);
-                // down: code, diagonal(s), b of level ls in; x and b of the others out (x of ls);
-                // up: code, diagonal(s), x, b in, x of ls out
-                const double dgs = (m == 2 ? 2 : 1) * m;
-                b += level == 0 ? n * (1 + dgs + (l == c->cmg_ls ? m : 0) + m + (l > c->cmg_ls ? m : 0))
-                                : n * (1 + dgs + 2 * m + (l == c->cmg_ls ? m : 0));
+                b += (double)lcells(l) * (1 + (l < c->lb ? m : 1) + (l == c->cmg_ls ? 2 * m : 0));
             }
             bpc = cells > 0 ? b / (double)cells : 0;
             break;
@@ -505,6 +523,11 @@ struct Run {
                                                            c->lv[l].split ? 1 : 0);
             end();
         }
+        if (c->cmg_ls > 0) {
+            beg(F_LEVEL, c->cmg_ls);
+            launch(k_cluster_lists<Pr>, c->cmg_cs, CL_THREADS, 0, s, cluster_args<M>(c, 0));
+            end();
+        }
         if (fork) cudaEventRecord(c->ev_join, c->aux);
         s = s0;
         const int64_t N = (int64_t)c->grid.n[0] * c->grid.n[1] * c->grid.n[2];
@@ -597,7 +620,7 @@ struct Run {
         down0.erase(down0.begin());
         for (int q = 0; q < swf; q++) { up0.push_back(1); up0.push_back(0); }
         const int lb = c->lb;
-        const int ls = c->cmg_ls > 0 ? c->cmg_ls : lb;  // levels ls .. lb-1 in the cluster
+        const int ls = c->cmg_ls > 0 ? c->cmg_ls : lb;  // levels ls .. L-1 in the cluster
         for (int l = 0; l < ls; l++) {
             if (l == 0 && with_start) start0();  // the coarser levels' starts ride on the restriction
             // b of the level's first pass waits for the preceding kernel where that kernel wrote
@@ -614,19 +637,9 @@ struct Run {
                 end();
             }
         }
-        BotArgs ba = c->bot;
-        ba.sweeps = sw;
-        ba.coarse = c->opts.coarse;
-        CmgArgs<M> ca;
         if (ls < lb) {
-            memset(&ca, 0, sizeof(ca));
-            ca.nl = lb - ls;
-            ca.sweeps = sw;
-            ca.botb = c->botb;
-            for (int l = ls; l <= lb; l++) ca.g[l - ls] = view<M>(c, l);
-            for (int l = ls; l < lb; l++) ca.s[l - ls] = c->cmg_slab[l - ls];
             beg(F_CMG, 0);
-            launch_cluster(k_cmg<Pr, 0>, c->cmg_cs, CMG_THREADS, c->cmg_smem, s, ca);
+            launch_cluster(k_cluster<Pr>, c->cmg_cs, CL_THREADS, c->cmg_smem, s, cluster_args<M>(c, sw));
             end();
         } else {
             const int64_t Nb = (int64_t)c->lv[lb].n[0] * c->lv[lb].n[1] * c->lv[lb].n[2];
@@ -634,13 +647,11 @@ struct Run {
             launch(k_restrict_bottom<Pr>, grid_cells(c, Nb), TPB, 0, s, view<M>(c, lb - 1), view<M>(c, lb),
                                                                     (typename Pr::C*)c->botb);
             end();
-        }
-        beg(F_BOTTOM, lb);
-        launch(k_bottom<Pr>, 1, 1024, c->bot_smem, s, (const typename Pr::C*)c->botb, (M*)c->lv[lb].x, ba);
-        end();
-        if (ls < lb) {
-            beg(F_CMG, 1);
-            launch_cluster(k_cmg<Pr, 1>, c->cmg_cs, CMG_THREADS, c->cmg_smem, s, ca);
+            BotArgs ba = c->bot;
+            ba.sweeps = sw;
+            ba.coarse = c->opts.coarse;
+            beg(F_BOTTOM, lb);
+            launch(k_bottom<Pr>, 1, 1024, c->bot_smem, s, (const typename Pr::C*)c->botb, (M*)c->lv[lb].x, ba);
             end();
         }
         for (int l = ls - 1; l >= 0; l--) {
@@ -861,21 +872,12 @@ struct GroupRun {
                        l + 1 < ls ? 1 : 0);
             }
         }
-        Grp<GCmg<M>> gc;
-        memset(&gc, 0, sizeof(gc));
         if (ls < lb) {
-            for (int i = 0; i < nb(); i++) {
-                mpp_ctx* ci = cs[i];
-                CmgArgs<M>& ca = gc.a[i].a;
-                ca.nl = lb - ls;
-                ca.sweeps = sw;
-                ca.botb = ci->botb;
-                for (int l = ls; l <= lb; l++) ca.g[l - ls] = view<M>(ci, l);
-                for (int l = ls; l < lb; l++) ca.s[l - ls] = ci->cmg_slab[l - ls];
-                gc.a[i].done = done_of(ci);
-            }
+            Grp<GCluster<M>> gc;
+            memset(&gc, 0, sizeof(gc));
+            for (int i = 0; i < nb(); i++) gc.a[i] = GCluster<M>{cluster_args<M>(cs[i], sw), done_of(cs[i])};
             nk++;
-            launch_clusters(k_cmg_g<Pr, 0>, c->cmg_cs, nb(), CMG_THREADS, c->cmg_smem, s, gc);
+            launch_clusters(k_cluster_g<Pr>, c->cmg_cs, nb(), CL_THREADS, c->cmg_smem, s, gc);
         } else {
             Grp<GRestrictBottom<M, C>> gr;
             memset(&gr, 0, sizeof(gr));
@@ -883,22 +885,17 @@ struct GroupRun {
                 gr.a[i] = GRestrictBottom<M, C>{view<M>(cs[i], lb - 1), view<M>(cs[i], lb), (C*)cs[i]->botb,
                                                 done_of(cs[i])};
             const int64_t Nb = (int64_t)c->lv[lb].n[0] * c->lv[lb].n[1] * c->lv[lb].n[2];
-            nk++;
+            Grp<GBottom<M, C>> gb;
+            memset(&gb, 0, sizeof(gb));
+            for (int i = 0; i < nb(); i++) {
+                BotArgs ba = cs[i]->bot;
+                ba.sweeps = sw;
+                ba.coarse = cs[i]->opts.coarse;
+                gb.a[i] = GBottom<M, C>{(const C*)cs[i]->botb, (M*)cs[i]->lv[lb].x, ba, done_of(cs[i])};
+            }
+            nk += 2;
             launch(k_restrict_bottom_g<Pr>, g2(grid_cells(c, Nb)), TPB, 0, s, gr);
-        }
-        Grp<GBottom<M, C>> gb;
-        memset(&gb, 0, sizeof(gb));
-        for (int i = 0; i < nb(); i++) {
-            BotArgs ba = cs[i]->bot;
-            ba.sweeps = sw;
-            ba.coarse = cs[i]->opts.coarse;
-            gb.a[i] = GBottom<M, C>{(const C*)cs[i]->botb, (M*)cs[i]->lv[lb].x, ba, done_of(cs[i])};
-        }
-        nk++;
-        launch(k_bottom_g<Pr>, g2(1), 1024, c->bot_smem, s, gb);
-        if (ls < lb) {
-            nk++;
-            launch_clusters(k_cmg_g<Pr, 1>, c->cmg_cs, nb(), CMG_THREADS, c->cmg_smem, s, gc);
+            launch(k_bottom_g<Pr>, g2(1), 1024, c->bot_smem, s, gb);
         }
         for (int l = ls - 1; l >= 0; l--) {
             nk++;
@@ -931,7 +928,7 @@ struct GroupRun {
         launch(k_group_cond, 1, 1, 0, s, d, nb(), cond);
     }
 };
-static_assert(sizeof(Grp<GCmg<double>>) < 32000, "a group launch's arguments fit the kernel parameter space");
+static_assert(sizeof(Grp<GCluster<double>>) < 32000, "a group launch's arguments fit the kernel parameter space");
 
 int write_params(mpp_ctx* c, float volume0, double dt, double recover, int project, float gamma, cudaStream_t s) {
     Params& p = c->sc_host->p;
@@ -1429,86 +1426,76 @@ bool encode_level(CUtensorMap* m, CUtensorMapDataType dt, void* base, size_t es,
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor maps for every row-split level whose rows are whole tiles (h extent a multiple of
-// 16, so every box start is 16-byte aligned) and whose j and k extents hold a halo box.
-// Levels without them, or with MPP_NO_TMA set in the environment, use k_rbgs.
-// The cluster-resident small levels: the lowest first level ls >= 1 of at most 32^3 cells
-// whose levels ls .. lb-1 fit, as z-slabs, in the shared memory of a cluster of 16 CTAs (8,
-// 4 or 2 when 16 does not divide their plane counts or does not run). In the environment
-// MPP_CMG=0 keeps the per-level launches, MPP_CMG_MAXCELLS sets the size bound and
-// MPP_CMG_CS the largest cluster.
+// The levels of k_cluster: from the first one of at most CL_CELLS cells whose planes (and those of
+// every smaller level) fit the shared memory of a cluster's CTAs, down to the coarsest. In the
+// environment MPP_CMG=0 keeps the per-level launches and MPP_CMG_MAXCELLS sets the size bound.
 int build_cmg(mpp_ctx* c) {
     c->cmg_ls = 0;
     c->cmg_cs = 0;
+    c->cmg_nd = c->cmg_nact = 0;
     c->cmg_smem = 0;
     const char* env = getenv("MPP_CMG");
     if ((env && !strcmp(env, "0")) || c->lb < 2) return MPP_OK;
-    // a level joins the cluster from this many cells down: 16 SMs run a pass over 32^3 cells
-    // in well under the latency of one launch over the whole GPU, over 64^3 cells they do not
-    int64_t maxcells = 32768;
+    int64_t maxcells = CL_CELLS;
     if (const char* mc = getenv("MPP_CMG_MAXCELLS")) maxcells = atoll(mc);
-    int csmax = 16;
-    if (const char* cm = getenv("MPP_CMG_CS")) csmax = atoi(cm);
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev));
-    const size_t ms = msize(c->prec);
-    const bool half = ms == 2;
+    const size_t cb = c->prec == MPP_PREC_FP64 ? 8 : 4;  // the arithmetic type
     return dispatch(c->prec, [&](auto pr) -> int {
         using Pr = decltype(pr);
-        cudaFuncAttributes fa0, fa1;
-        CK(cudaFuncGetAttributes(&fa0, k_cmg<Pr, 0>));
-        CK(cudaFuncGetAttributes(&fa1, k_cmg<Pr, 1>));
-        const size_t stat = fa0.sharedSizeBytes > fa1.sharedSizeBytes ? fa0.sharedSizeBytes : fa1.sharedSizeBytes;
+        cudaFuncAttributes fa;
+        CK(cudaFuncGetAttributes(&fa, k_cluster<Pr>));
+        const size_t stat = fa.sharedSizeBytes;
+        auto cells = [&](int l) { return (int64_t)c->lv[l].n[0] * c->lv[l].n[1] * c->lv[l].n[2]; };
         for (int ls = 1; ls < c->lb; ls++) {
-            if (c->lb - ls > CMG_MAXLEV) continue;
-            if ((int64_t)c->lv[ls].n[0] * c->lv[ls].n[1] * c->lv[ls].n[2] > maxcells) continue;
-            for (int cs : {16, 8, 4, 2}) {
-                if (cs > csmax) continue;
+            const int nl = c->L - 1 - ls;
+            if (nl > CL_MAXLEV || cells(ls) > maxcells) continue;
+            int nd = 0;
+            while (nd < nl && cells(ls + nd) > CL_LOCAL_CELLS) nd++;
+            if (nd == nl) continue;  // (the level above the coarsest has at most 8 x 1024 cells)
+            for (int cs : {CL_SIZE, CL_SIZE / 2}) {
+                if (nd == 0) cs = 1;
+                ClLev lev[CL_MAXLEV + 1];
+                memset(lev, 0, sizeof(lev));
+                size_t off = 0;
+                int ngent = 0;
                 bool ok = true;
-                size_t off = CMG_HEADER;  // the active-row counts
-                CmgSlab sl[CMG_MAXLEV];
                 auto take = [&](size_t bytes) {
                     const unsigned o = (unsigned)off;
                     off += (bytes + 15) / 16 * 16;
                     return o;
                 };
-                for (int l = ls; l < c->lb && ok; l++) {
-                    const LevelBuf& b = c->lv[l];
-                    if (!b.split || b.n[0] % 2 || b.n[0] < 4 || b.n[2] % cs || b.n[1] > 65535) {
-                        ok = false;
-                        break;
-                    }
-                    CmgSlab& S = sl[l - ls];
+                // the top level's planes a CTA: whole planes of every spread level's, down to one
+                const int unit = 1 << nd, n3 = c->lv[ls].n[2], P0 = unit * ((n3 / unit + cs - 1) / cs);
+                for (int q = 0; q <= nl && ok; q++) {
+                    const LevelBuf& b = c->lv[ls + q];
+                    ClLev& S = lev[q];
                     S.n1 = b.n[0];
                     S.n2 = b.n[1];
                     S.n3 = b.n[2];
-                    S.P = b.n[2] / cs;
-                    S.H = S.n1 / 2;
-                    auto magic = [](int d) { return d > 1 ? 0xFFFFFFFFu / (unsigned)d + 1u : 0u; };
-                    S.mH = magic(S.H);
-                    S.mN = magic(S.n1);
-                    S.mP = magic(S.P);
-                    const size_t n = (size_t)S.P * S.n1 * S.n2;
-                    if (n >= 65536) {  // items of a pass are counted in 16 bits
-                        ok = false;
-                        break;
-                    }
-                    S.ox = take(ms * n);
-                    S.ob = take(ms * n);
-                    S.orr = take(ms * n);
-                    S.ocode = take(n);
-                    S.odg = take(ms * n);
-                    S.odi = half ? take(ms * n) : 0;
-                    S.orows = take(sizeof(uint32_t) * (size_t)S.P * S.n2);
+                    S.P = q < nd ? P0 >> q : S.n3;
+                    S.RS = (S.n1 + 1) / 2 + 1;
+                    S.PS = (S.n2 + 1) * S.RS;
+                    S.CS = (S.P + 2) * S.PS + S.RS + 1;
+                    S.cap = S.P * S.n2 * ((S.n1 + 1) / 2);
+                    S.full = ls + q >= c->lb ? 1 : 0;
+                    if (S.CS >= 65536 || (q < nl && S.n1 % 2)) ok = false;  // a place is 16 bits
+                    S.ox = take(cb * 2 * S.CS);
+                    if (q == nl) break;
+                    S.ob = take(cb * 2 * S.CS);
+                    S.orr = take(cb * 2 * S.CS);
+                    S.oent = take(sizeof(uint2) * 2 * (size_t)S.cap);
+                    S.gent = ngent;
+                    ngent += 2 * S.cap * (q < nd ? cs : 1);
                 }
-                if (!ok || off + stat > (size_t)optin) continue;
-                for (auto kern : {k_cmg<Pr, 0>, k_cmg<Pr, 1>}) {  // the limit is the function's: the device's
-                    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)stat));
-                    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-                }
+                const unsigned orb = take(sizeof(uint4) * 2 * RB_HALF);
+                const unsigned ogi = take(sizeof(uint32_t) * 2 * (size_t)lev[0].cap);
+                if (!ok || off + stat > (size_t)optin) break;  // (half the cluster holds twice the planes)
+                CK(cudaFuncSetAttribute(k_cluster<Pr>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)stat));
+                CK(cudaFuncSetAttribute(k_cluster<Pr>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3((unsigned)cs);
-                cfg.blockDim = dim3((unsigned)CMG_THREADS);
+                cfg.blockDim = dim3((unsigned)CL_THREADS);
                 cfg.dynamicSmemBytes = off;
                 cudaLaunchAttribute at[1];
                 at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1518,15 +1505,26 @@ int build_cmg(mpp_ctx* c) {
                 cfg.attrs = at;
                 cfg.numAttrs = 1;
                 int nc = 0;
-                if (cudaOccupancyMaxActiveClusters(&nc, k_cmg<Pr, 0>, &cfg) != cudaSuccess) {
+                if (cudaOccupancyMaxActiveClusters(&nc, k_cluster<Pr>, &cfg) != cudaSuccess) {
                     cudaGetLastError();
-                    continue;
+                    nc = 0;
                 }
                 if (nc < 1) continue;
+                ClLists& l = c->cmg_l;
+                if (int e = alloc(c, (void**)&l.ent, sizeof(uint2) * (size_t)ngent)) return e;
+                if (int e = alloc(c, (void**)&l.gidx, sizeof(uint32_t) * 2 * (size_t)lev[0].cap * cs)) return e;
+                if (int e = alloc(c, (void**)&l.cnt, sizeof(int4) * CL_MAXLEV * CL_SIZE)) return e;
+                if (int e = alloc(c, (void**)&l.rb, sizeof(uint4) * 2 * RB_HALF)) return e;
+                if (int e = alloc(c, (void**)&l.nrb, sizeof(int) * 2)) return e;
+                if (int e = alloc(c, &l.share, cb * 2 * (size_t)lev[nd].CS + 16)) return e;
                 c->cmg_ls = ls;
                 c->cmg_cs = cs;
+                c->cmg_nd = nd;
+                c->cmg_nact = nd > 0 ? (n3 + P0 - 1) / P0 : 1;
                 c->cmg_smem = off;
-                for (int l = ls; l < c->lb; l++) c->cmg_slab[l - ls] = sl[l - ls];
+                c->cmg_orb = orb;
+                c->cmg_ogi = ogi;
+                memcpy(c->cmg_lev, lev, sizeof(lev));
                 return MPP_OK;
             }
         }
@@ -1534,6 +1532,9 @@ int build_cmg(mpp_ctx* c) {
     });
 }
 
+// Tensor maps for every row-split level whose rows are whole tiles (h extent a multiple of
+// 16, so every box start is 16-byte aligned) and whose j and k extents hold a halo box.
+// Levels without them, or with MPP_NO_TMA set in the environment, use k_rbgs.
 int build_tma(mpp_ctx* c) {
     const size_t ms = msize(c->prec);
     const CUtensorMapDataType dt = c->prec == MPP_PREC_FP64        ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
@@ -1734,8 +1735,7 @@ int mpp_ctx_create(mpp_ctx** out, const mpp_grid* g, const mpp_opts* o) {
     // level geometry
     size_t tflag_total = 0;
     // the first level small enough for the one-CTA bottom solve: 4096 cells, or 512 when the
-    // levels above it can run in a thread-block cluster (k_cmg takes a 16^3 level's passes in
-    // well under the time one CTA needs); MPP_BOTTOM_CELLS in the environment lowers the bound
+    // levels above it can run in k_cluster; MPP_BOTTOM_CELLS in the environment lowers the bound
     const char* cmg_env = getenv("MPP_CMG");
     int64_t botcells = (cmg_env && !strcmp(cmg_env, "0")) ? BOTTOM_CELLS : BOTTOM_CELLS / 8;
     if (const char* bc = getenv("MPP_BOTTOM_CELLS")) botcells = std::min<int64_t>(BOTTOM_CELLS, atoll(bc));
@@ -2048,7 +2048,7 @@ int group_attrs(const mpp_ctx* c) {
     CK(cudaFuncGetAttributes(&fb, k_bottom_g<Pr>));  // its static part (the list counts)
     CK(cudaFuncSetAttribute(k_bottom_g<Pr>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fb.sharedSizeBytes));
     CK(cudaFuncSetAttribute(k_restrict_g<Pr>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->restrict_smem));
-    for (auto kern : {k_cmg_g<Pr, 0>, k_cmg_g<Pr, 1>}) {
+    for (auto kern : {k_cluster_g<Pr>}) {
         cudaFuncAttributes fa;
         CK(cudaFuncGetAttributes(&fa, kern));
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));

@@ -10,7 +10,7 @@
 // is done.
 #pragma once
 
-#include "mpp_cmg.cuh"
+#include "mpp_cluster.cuh"
 #include "mpp_tma.cuh"
 
 namespace mpp {
@@ -41,8 +41,8 @@ struct GRestrictBottom {
     const int* done;
 };
 template <class M>
-struct GCmg {
-    CmgArgs<M> a;
+struct GCluster {
+    ClArgs<M> a;
     const int* done;
 };
 template <class M, class C>
@@ -130,11 +130,11 @@ __global__ void __launch_bounds__(TPB)
     if (grp_skip(a.done)) return;
     restrict_bottom_dev<Pr>(a.F, a.L, a.bout);
 }
-template <class Pr, int UP>
-__global__ void __launch_bounds__(CMG_THREADS, 1) k_cmg_g(const __grid_constant__ Grp<GCmg<typename Pr::M>> g) {
+template <class Pr>
+__global__ void __launch_bounds__(CL_THREADS, 1) k_cluster_g(const __grid_constant__ Grp<GCluster<typename Pr::M>> g) {
     const auto& a = g.a[blockIdx.y];
     if (grp_skip(a.done)) return;  // every CTA of the basin's cluster returns together
-    cmg_dev<Pr, UP>(a.a);
+    cluster_dev<Pr>(a.a);
 }
 template <class Pr>
 __global__ void __launch_bounds__(1024)

@@ -15,6 +15,7 @@
 #pragma once
 
 #include "mpp_base.cuh"
+#include "mpp_coarsest.cuh"
 
 namespace mpp {
 
@@ -499,15 +500,90 @@ struct BotArgs {
     BotLev lv[BOTTOM_MAXLEV];
 };
 
+// The coarsest level's lists of unknowns (a cell with no open face stays 0).
+template <class Pr>
+__device__ __forceinline__ int coarsest_lists(const BotLev& B, RbShared<typename Pr::CC>& sh) {
+    return rb_lists<typename Pr::CC>(
+        sh, B.n1 * B.n2 * B.n3, [&](int c) { return (B.code[c] & SELF) && B.dc[c] > 0; },
+        [&](int c) { return (c % B.n1 + (c / B.n1) % B.n2 + c / (B.n1 * B.n2) + 1) & 1; });
+}
+// coarse_kernel! on level B (at most 1024 cells; a block of at least as many threads, the lists
+// built): getb(c) is a cell's right-hand side, put(c, x) takes every cell's result, once.
+// wait: the right-hand side is the preceding kernel's output.
+template <class Pr, class GetB, class Put>
+__device__ __forceinline__ void coarsest_solve(const BotLev& B, int sweeps, RbShared<typename Pr::CC>& sh, int nt,
+                                               GetB&& getb, Put&& put, bool wait = false) {
+    using CC = typename Pr::CC;
+    const int tid = (int)threadIdx.x, N = B.n1 * B.n2 * B.n3;
+    const int step6[6] = {1, -1, B.n1, -B.n1, B.n1 * B.n2, -B.n1 * B.n2};
+    int own[2], nb[2][6], cell[2];
+    CC bi[2], d[2], rd[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        own[u] = RB_CELLS + 1;  // a thread without an unknown solves 0 = 0 into a spare place
+        cell[u] = -1;
+        bi[u] = (CC)0;
+        d[u] = rd[u] = (CC)1;
+#pragma unroll
+        for (int m = 0; m < 6; m++) nb[u][m] = RB_CELLS;
+        if (tid < sh.cnt[u][32]) {
+            const int c = sh.cell[u][tid];
+            const uint8_t cd = B.code[c];
+            cell[u] = c;
+            own[u] = u * RB_HALF + tid;
+            d[u] = (CC)B.dc[c];
+            rd[u] = (CC)1 / d[u];
+#pragma unroll
+            for (int m = 0; m < 6; m++)
+                if (cd & (1u << m)) nb[u][m] = sh.place[c + step6[m]];
+        }
+    }
+    if (wait) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    if (tid < nt) {
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+            if (cell[u] >= 0) bi[u] = getb(cell[u]);
+        rb_sweeps(nt, sweeps, [&](auto uc) {
+            constexpr int u = decltype(uc)::value;
+            CC v[6];
+#pragma unroll
+            for (int m = 0; m < 6; m++) v[m] = sh.x[nb[u][m]];
+            CC acc = bi[u];
+#pragma unroll
+            for (int m = 0; m < 6; m++) acc += v[m];  // (a neighbour that is no unknown adds 0)
+            if constexpr (std::is_same<CC, float>::value) sh.x[own[u]] = div_small(acc, d[u], rd[u]);
+            else sh.x[own[u]] = acc * rd[u];  // FP64 coarsest of the 16-bit forms
+        });
+    }
+    __syncthreads();
+    for (int c = tid; c < N; c += (int)blockDim.x) put(c, sh.x[sh.place[c]]);
+}
+
 template <class Pr>
 __device__ __forceinline__ void bottom_dev(const typename Pr::C* __restrict__ bin, typename Pr::M* __restrict__ xout,
                                            const BotArgs& a) {
-    pdl_wait();
-    pdl_trigger();
     using C = typename Pr::C;
     using CC = typename Pr::CC;
     extern __shared__ __align__(128) unsigned char smraw[];
     const int T = blockDim.x, tid = threadIdx.x;
+    // the coarsest level's lists of unknowns: its codes date from the set-up, so they are read
+    // before the programmatic-dependent-launch wait
+    __shared__ RbShared<CC> rb;
+    int rb_threads;
+    {
+        const BotLev& B = a.lv[a.nl - 1];
+        rb_threads = coarsest_lists<Pr>(B, rb);
+    }
+    if (a.nl == 1) {  // the usual case: the coarsest level is the only one here
+        coarsest_solve<Pr>(a.lv[0], a.coarse, rb, rb_threads,
+                           [&](int c) { return (CC)bin[c]; }, [&](int c, CC v) { st(xout + c, v); }, true);
+        return;
+    }
+    pdl_wait();
+    pdl_trigger();
     // codes and non-SOLID neighbour counts of every level, and level lb's right-hand side
     // (restricted from the level above by k_restrict_bottom)
     // per level above the coarsest: its LIQUID cells listed by colour (the red-black passes
@@ -535,13 +611,8 @@ __device__ __forceinline__ void bottom_dev(const typename Pr::C* __restrict__ bi
     {
         const BotLev& B = a.lv[0];
         const int N = B.n1 * B.n2 * B.n3;
-        if (a.nl == 1) {
-            CC* b = reinterpret_cast<CC*>(smraw + B.ob);
-            for (int c = tid; c < N; c += T) b[c] = (CC)bin[c];
-        } else {
-            C* b = reinterpret_cast<C*>(smraw + B.ob);
-            for (int c = tid; c < N; c += T) b[c] = bin[c];
-        }
+        C* b = reinterpret_cast<C*>(smraw + B.ob);
+        for (int c = tid; c < N; c += T) b[c] = bin[c];
     }
     __syncthreads();
     // restriction between shared-memory levels
@@ -643,65 +714,11 @@ __device__ __forceinline__ void bottom_dev(const typename Pr::C* __restrict__ bi
         else restrict_into(l + 1, reinterpret_cast<C*>(smraw + a.lv[l + 1].ob), getL);
         __syncthreads();
     }
-    {  // coarse_kernel!
-        const BotLev& B = a.lv[a.nl - 1];
-        const int N = B.n1 * B.n2 * B.n3, sy = B.n1, sz = B.n1 * B.n2;
-        const uint8_t* code = smraw + B.ocode;
-        const uint8_t* dc = smraw + B.odc;
-        CC* x = reinterpret_cast<CC*>(smraw + B.ox);
-        const CC* b = reinterpret_cast<const CC*>(smraw + B.ob);
-        for (int c = tid; c < N; c += T) x[c] = (CC)0;
-        __syncthreads();
-        // With n1 even a thread owns cells 2t and 2t+1 of one row, one of each colour, and each
-        // half-sweep updates the one of that colour (selected without branching); with n1 odd,
-        // one cell per thread. Only the threads that own cells meet at each barrier.
-        const int per = (B.n1 % 2 == 0) ? 2 : 1;
-        const int nthreads = (((N + per - 1) / per + 31) / 32) * 32;
-        if (tid < nthreads) {
-            uint8_t cd[2] = {0, 0};
-            int cell[2] = {0, 0};
-            CC bi[2] = {(CC)0, (CC)0}, d[2] = {(CC)0, (CC)0}, rd[2] = {(CC)0, (CC)0};
-            int col0 = 0;
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int c = per * tid + u;
-                cell[u] = c;
-                if (u < per && c < N) {
-                    cd[u] = code[c];
-                    const int i = c % B.n1, j = (c / B.n1) % B.n2, k = c / sz;
-                    if (u == 0) col0 = (i + j + k + 1) & 1;
-                    bi[u] = b[c];
-                    d[u] = (CC)dc[c];
-                    rd[u] = d[u] > (CC)0 ? (CC)1 / d[u] : (CC)0;
-                }
-            }
-            for (int s = 1; s <= 2 * a.coarse; s++)
-                for (int half = 0; half <= 1; half++) {
-                    const int colour = s <= a.coarse ? half : 1 - half;
-                    // this thread's cell of `colour` (per == 1: its only cell, if that colour)
-                    const bool second = per == 2 && col0 != colour;
-                    const uint8_t cdv = (per == 1 && col0 != colour) ? (uint8_t)0 : (second ? cd[1] : cd[0]);
-                    if (cdv & SELF) {
-                        const int c = second ? cell[1] : cell[0];
-                        CC acc = second ? bi[1] : bi[0];
-                        if (cdv & 1) acc += x[c + 1];
-                        if (cdv & 2) acc += x[c - 1];
-                        if (cdv & 4) acc += x[c + sy];
-                        if (cdv & 8) acc += x[c - sy];
-                        if (cdv & 16) acc += x[c + sz];
-                        if (cdv & 32) acc += x[c - sz];
-                        if constexpr (std::is_same<CC, float>::value) {
-                            const CC dd = second ? d[1] : d[0];
-                            x[c] = dd > (CC)0 ? acc / dd : (CC)0;
-                        } else {
-                            x[c] = acc * (second ? rd[1] : rd[0]);  // FP64 coarsest of the 16-bit forms
-                        }
-                    }
-                    asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
-                }
-        }
-        __syncthreads();
-    }
+    // coarse_kernel!
+    coarsest_solve<Pr>(a.lv[a.nl - 1], a.coarse, rb, rb_threads,
+                       [&](int c) { return reinterpret_cast<const CC*>(smraw + a.lv[a.nl - 1].ob)[c]; },
+                       [&](int c, CC v) { reinterpret_cast<CC*>(smraw + a.lv[a.nl - 1].ox)[c] = v; });
+    __syncthreads();
     // back up: prolongation and the up sweeps
     for (int l = a.nl - 2; l >= 0; l--) {
         const BotLev& B = a.lv[l];
@@ -742,13 +759,8 @@ __device__ __forceinline__ void bottom_dev(const typename Pr::C* __restrict__ bi
     {
         const BotLev& B = a.lv[0];
         const int N = B.n1 * B.n2 * B.n3;
-        if (a.nl == 1) {
-            const CC* x = reinterpret_cast<const CC*>(smraw + B.ox);
-            for (int c = tid; c < N; c += T) st(xout + c, x[c]);
-        } else {
-            const C* x = reinterpret_cast<const C*>(smraw + B.ox);
-            for (int c = tid; c < N; c += T) st(xout + c, x[c]);
-        }
+        const C* x = reinterpret_cast<const C*>(smraw + B.ox);
+        for (int c = tid; c < N; c += T) st(xout + c, x[c]);
     }
 }
 template <class Pr>
