@@ -208,29 +208,28 @@ __global__ void __launch_bounds__(SPT, 6) k_sp_blk(Topo t, Comp L, const uint16_
         });
     } else {
         constexpr bool ZS = OP == BOP_JAC_ZS;
-        SP_ACTIVE_LOOP(c, L, gf) {
-            int I, J, K;
-            coarse_cell(t, c, I, J, K);
-            float diag, off;
-            coarserow_s<16, ZS>(t, L, src, I, J, K, diag, off);
-            const float x0 = ZS ? 0.0f : src.coarse(c);
+        coarse_rows<16, ZS>(t, L, src, gf, [&](int64_t c, float off) {
+            const float x0 = ZS ? 0.0f : src.coarse(c), diag = L.dgc[c];
             float v;
             if (OP == BOP_RES) v = bc[c] - (diag * x0 - off);
             else v = diag > 0.0f ? x0 + OMEGA * (bc[c] - (diag * x0 - off)) / diag : 0.0f;
             outc[c] = v;
-        }
+        });
     }
 }
 
-// The coarse unknowns' whole diagonals (coarserow's sums), for SrcZS.
+// The coarse unknowns' whole diagonals at a level (coarserow's sums).
+template <int N>
 __global__ void __launch_bounds__(SPT) k_sp_dgc(Topo t, Comp L, float* dgc) {
     pdl_wait();
     pdl_trigger();
-    SP_ACTIVE_LOOP(c, L, 0) {
+    const int nin = L.nclist[0], n = nin + L.nclist[1];
+    for (int e = (int)blockIdx.x * (int)blockDim.x + (int)threadIdx.x; e < n; e += (int)gridDim.x * (int)blockDim.x) {
+        const int c = L.clist[e < nin ? e : L.ncc - 1 - (e - nin)];
         int I, J, K;
         coarse_cell(t, c, I, J, K);
         float diag, off;
-        coarserow<16, true>(t, L, nullptr, nullptr, I, J, K, diag, off);
+        coarserow<N, true>(t, L, nullptr, nullptr, I, J, K, diag, off);
         dgc[c] = diag;
     }
 }
@@ -360,15 +359,11 @@ __global__ void __launch_bounds__(SPT, 6) k_sp_apply_dot(Topo t, Comp L, const u
                                 ldm4(tf + n), LIQUID);
             });
     } else {
-        SP_ACTIVE_LOOP(c, L, gf) {
-            int I, J, K;
-            coarse_cell(t, c, I, J, K);
-            float diag, off;
-            coarserow<16, false>(t, L, df, dc, I, J, K, diag, off);
-            const float q = diag * dc[c] - off;
+        coarse_rows<16, false>(t, L, SrcX{df, dc}, gf, [&](int64_t c, float off) {
+            const float q = L.dgc[c] * dc[c] - off;
             qc[c] = q;
             acc[0] += (double)dc[c] * (double)q;
-        }
+        });
     }
     if (grid_sum<1>(acc, partials, counter) && threadIdx.x == 0) {
         const float den = (float)acc[0];
@@ -544,13 +539,8 @@ __global__ void __launch_bounds__(SPT) k_sp_apply(Topo t, Comp L, const uint16_t
             st4(qf + n, make_float4(q[0], q[1], q[2], q[3]));
         });
     } else {
-        SP_ACTIVE_LOOP(c, L, gf) {
-            int I, J, K;
-            coarse_cell(t, c, I, J, K);
-            float diag, off;
-            coarserow<16, false>(t, L, xf, xc, I, J, K, diag, off);
-            qc[c] = diag * xc[c] - off;
-        }
+        coarse_rows<16, false>(t, L, SrcX{xf, xc}, gf,
+                               [&](int64_t c, float off) { qc[c] = L.dgc[c] * xc[c] - off; });
     }
 }
 // a.b over the unknowns (inner), FP64, into *out
@@ -710,8 +700,9 @@ struct mpp_sparse_ctx {
     uint16_t* code0;    // each fine cell's six couplings, active and LIQUID bits (the block kernels)
     float* dg0;         // each fine cell's whole diagonal
     uint8_t* cmask;     // the coarse unknowns (LIQUID, no fine block over them)
-    float* dgc;         // and their whole diagonals
-    int* clist;         // and their indices, listed by the operator (nclist of them)
+    uint8_t* ccode;     // which of their coarse neighbours couple
+    float *dgc, *dgc1;  // and their whole diagonals at levels 0 and 1
+    int* clist;         // and their indices, listed by the operator (nclist: see Comp)
     int* nclist;
     uint8_t* actc;      // = D[0].act
     // level 1
@@ -805,14 +796,14 @@ Comp comp0(const mpp_sparse_ctx* c, const uint8_t* tf) {
     Comp L;
     L.cfx = c->cf[0]; L.cfy = c->cf[1]; L.cfz = c->cf[2]; L.dDf = c->dDf; L.actf = tf;
     L.ccx = c->cc[0]; L.ccy = c->cc[1]; L.ccz = c->cc[2]; L.dDc = c->dDc; L.actc = c->actc;
-    L.clist = c->clist; L.nclist = c->nclist;
+    L.clist = c->clist; L.nclist = c->nclist; L.ncc = (int)c->ncc; L.ccode = c->ccode; L.dgc = c->dgc;
     return L;
 }
 Comp comp1(const mpp_sparse_ctx* c) {
     Comp L;
     L.cfx = c->c1[0]; L.cfy = c->c1[1]; L.cfz = c->c1[2]; L.dDf = c->dD1; L.actf = c->act1;
     L.ccx = c->cc[0]; L.ccy = c->cc[1]; L.ccz = c->cc[2]; L.dDc = c->dDc; L.actc = c->actc;
-    L.clist = c->clist; L.nclist = c->nclist;
+    L.clist = c->clist; L.nclist = c->nclist; L.ncc = (int)c->ncc; L.ccode = c->ccode; L.dgc = c->dgc1;
     return L;
 }
 
@@ -854,14 +845,14 @@ struct SpRun {
         for (int a = 1; a <= 3; a++) mc = std::max(mc, face_count(t.nc, a));
         sp_launch(k_sp_coarsecoef, dim3(grid1(mc), 3), SPT, s, t, c->cc[0], c->cc[1], c->cc[2], b->types_c);
         const Split sp = split_for(c, (int64_t)t.nslots * BCELLS);
-        cudaMemsetAsync(c->nclist, 0, sizeof(int), s);
+        cudaMemsetAsync(c->nclist, 0, 2 * sizeof(int), s);
         // the coarse parts the composite passes write only on the listed cells start at zero
         for (float* a : {c->tmc, c->zc, c->res0c, c->qc, c->t1c, c->x1c, c->r1c})
             cudaMemsetAsync(a, 0, sizeof(float) * (size_t)c->ncc, s);
         sp_launch(k_sp_dirichlet, dim3(sp.g), SPT, s, t, c->dDf, c->dDc, c->actc, b->types_f, b->types_c, b->phi_f,
                   b->phi_c, (const float*)c->cf[0], (const float*)c->cf[1], (const float*)c->cf[2], c->code0, c->dg0,
-                  c->cmask, c->clist, c->nclist, sp.gf);
-        sp_launch(k_sp_dgc, dim3(cap_blocks(c, c->ncc)), SPT, s, t, comp0(c, b->types_f), c->dgc);
+                  c->cmask, c->clist, c->nclist, c->ccode, sp.gf);
+        sp_launch(k_sp_dgc<16>, dim3(cap_blocks(c, c->ncc)), SPT, s, t, comp0(c, b->types_f), c->dgc);
         nk += 4;
         hierarchy(b->types_f);
     }
@@ -872,6 +863,8 @@ struct SpRun {
         sp_launch(k_sp_cells1, dim3(grid1((int64_t)t.nslots * BCELLS1)), SPT, s, t, c->dD1, c->act1,
                   (const float*)c->dDf, tf, (const float*)c->c1[0], (const float*)c->c1[1], (const float*)c->c1[2],
                   c->dg1);
+        sp_launch(k_sp_dgc<8>, dim3(cap_blocks(c, c->ncc)), SPT, s, t, comp1(c), c->dgc1);
+        nk++;
         int64_t mc = c->ncc;
         for (int a = 1; a <= 3; a++) mc = std::max(mc, face_count(t.nc, a));
         sp_launch(k_sp_level2, dim3(grid1(mc), 4), SPT, s, t, c->D[0].cx, c->D[0].cy, c->D[0].cz,
@@ -1398,7 +1391,9 @@ int mpp_sparse_ctx_create(mpp_sparse_ctx** out, const mpp_sparse_grid* g, int32_
     if (!e) e = sp_alloc_n(c, &c->dg0, nf);
     if (!e) e = sp_alloc_n(c, &c->cmask, c->ncc);
     if (!e) e = sp_alloc_n(c, &c->clist, c->ncc);
-    if (!e) e = sp_alloc_n(c, &c->nclist, 1);
+    if (!e) e = sp_alloc_n(c, &c->nclist, 2);
+    if (!e) e = sp_alloc_n(c, &c->ccode, c->ncc);
+    if (!e) e = sp_alloc_n(c, &c->dgc1, c->ncc);
     int m[3] = {c->t.nc[0], c->t.nc[1], c->t.nc[2]};
     for (int l = 0; l < nd && !e; l++) {
         DL& D = c->D[l];

@@ -163,10 +163,15 @@ struct Comp {
     const float *ccx, *ccy, *ccz, *dDc;
     const uint8_t* actc;
     // the coarse cells the composite passes update (LIQUID, no fine block over them; actc is
-    // set on exactly these outside fine blocks), listed once per operator: the passes walk
-    // the list, and every other coarse cell of their outputs stays at the zero it was cleared to
+    // set on exactly these outside fine blocks), listed once per operator: those with no fine block
+    // beside them from the list's front (nclist[0]), the others from its back (nclist[1]). The
+    // passes walk the list, and every other coarse cell of their outputs stays at the zero it was
+    // cleared to.
     const int* clist;
     const int* nclist;
+    int ncc;               // the list's places
+    const uint8_t* ccode;  // which coarse neighbours couple (bits in coarserow's order, COARSE_COARSE each)
+    const float* dgc;      // the whole diagonal at this level, coarserow's sums
 };
 
 // Where a level-0 pass reads x: the stored values (SrcX), or values formed on the fly, with
@@ -327,15 +332,101 @@ __device__ __forceinline__ int sp_slot(int gf) { return (int)blockIdx.x - ((int)
 #define SP_FINE_LOOP(n, total, gf)                                                                        \
     for (int64_t n = (int64_t)((int)blockIdx.x - ((int)gridDim.x - (gf))) * blockDim.x + threadIdx.x; n < (total); \
          n += (int64_t)(gf) * blockDim.x)
-// The coarse part's walk over the operator's list of coarse unknowns (the coarse CTAs of a
-// fused launch, [0, gridDim - gf), as SP_COARSE_LOOP).
-#define SP_ACTIVE_LOOP(c, L, gf)                                                                   \
-    for (int64_t e_ = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ne_ = *(L).nclist; e_ < ne_; \
-         e_ += (int64_t)(gridDim.x - (gf)) * blockDim.x)                                           \
-        if (const int64_t c = (L).clist[e_]; true)
 #define SP_COARSE_LOOP(c, total, gf)                                                               \
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < (total);                  \
          c += (int64_t)(gridDim.x - (gf)) * blockDim.x)
+
+// The coarse part of a composite pass: f(c, off) once for every coarse unknown, off being
+// coarserow's sum (its diagonal is L.dgc[c]); the coarse CTAs of a fused launch, [0, gridDim - gf).
+// ZS: x is zero everywhere.
+// A cell beside fine blocks reads R^2 sub-faces and as many fine cells a direction. A thread that
+// walked them one after the other was the whole launch's time on a small basin (sweeps of 87 slots:
+// 30 us with SrcZS, 24 with SrcPro, 9 with SrcX; now 10, 9 and 7; 2948 slots: 83, 75 and 62 us, now
+// 77, 69 and 58). A group of R^2 lanes takes such a cell: the six
+// directions' blocks are looked up by six lanes at once, a lane loads its sub-face's coupling and
+// cell for every direction, and the products are added in coarserow's order by a shuffle each. The
+// other cells, most of them, are seven loads around a byte of couplings, a thread each.
+template <int N, bool ZS, class Src, class F>
+__device__ __forceinline__ void coarse_rows(const Topo& t, const Comp& L, const Src& src, int gf, F&& f) {
+    using V = Lv<N>;
+    constexpr int R = N / 4, G = R * R, M = N - 1;
+    const int n1 = t.nc[0], n2 = t.nc[1], n3 = t.nc[2], ctas = (int)gridDim.x - gf;
+    const int nin = L.nclist[0], nedge = L.nclist[1];
+    const int g = (int)threadIdx.x & (G - 1), per = (int)blockDim.x / G, wg = 32 / G;
+    const int first = ((int)blockIdx.x * per + ((int)threadIdx.x >> 5) * wg), mine = ((int)threadIdx.x & 31) / G;
+    for (int e0 = first; e0 < nedge; e0 += ctas * per) {  // (a warp's groups go round together)
+        const bool is = e0 + mine < nedge;
+        const int c = L.clist[L.ncc - 1 - (is ? e0 + mine : e0)];
+        int I, J, K;
+        split3(c, n1, n2, I, J, K);
+        const unsigned cc = L.ccode[c];
+        // lane g looks up direction g (and g + G where the group has fewer than six lanes)
+        int look[(6 + G - 1) / G];
+#pragma unroll
+        for (int u = 0; u < (6 + G - 1) / G; u++) {
+            const int d = g + u * G, a = d >> 1, sg = (d & 1) ? 1 : -1;
+            look[u] = 0;
+            if (d < 6) {
+                const int In = I + (a == 0 ? sg : 0), Jn = J + (a == 1 ? sg : 0), Kn = K + (a == 2 ? sg : 0);
+                if (0 <= In && In < n1 && 0 <= Jn && Jn < n2 && 0 <= Kn && Kn < n3)
+                    look[u] = cellslot(t, In * RATIO, Jn * RATIO, Kn * RATIO);
+            }
+        }
+        const int q = g / R, p = g % R;  // this lane's sub-face
+        int slot[6];
+        float v[6];
+#pragma unroll
+        for (int d = 0; d < 6; d++) {
+            const int s2 = __shfl_sync(0xffffffffu, look[d / G], d % G, G);
+            const int a = d >> 1, sg = (d & 1) ? 1 : -1;
+            slot[d] = s2;
+            v[d] = 0.0f;
+            if (ZS) continue;
+            if (s2 != 0) {
+                // the sub-face is in block s2: its cell's low face (sg > 0), or the block's high plane
+                const int fi = a == 0 ? (sg > 0 ? 0 : M) : (R * I + p) & M;
+                const int fj = a == 1 ? (sg > 0 ? 0 : M) : (R * J + (a == 0 ? p : q)) & M;
+                const int fk = a == 2 ? (sg > 0 ? 0 : M) : (R * K + q) & M;
+                const float* Cf = a == 0 ? L.cfx : (a == 1 ? L.cfy : L.cfz);
+                const float w = Cf[V::face(s2, a + 1, a == 0 && sg < 0 ? N : fi, a == 1 && sg < 0 ? N : fj,
+                                           a == 2 && sg < 0 ? N : fk) - 1];
+                v[d] = w * src.fine(V::cell(s2, fi, fj, fk) - 1);
+            } else if (cc & (1u << d)) {
+                v[d] = COARSE_COARSE * src.coarse(c + sg * (a == 0 ? 1 : (a == 1 ? n1 : n1 * n2)));
+            }
+        }
+        float off = 0.0f;
+        if (!ZS) {
+#pragma unroll
+            for (int d = 0; d < 6; d++) {
+                if (__any_sync(0xffffffffu, slot[d] != 0)) {
+#pragma unroll
+                    for (int i = 0; i < G; i++) {
+                        const float x = __shfl_sync(0xffffffffu, v[d], i, G);
+                        if (slot[d] != 0) off += x;
+                    }
+                }
+                if (slot[d] == 0 && (cc & (1u << d))) off += v[d];
+            }
+        }
+        if (is && g == 0) f((int64_t)c, off);
+    }
+    for (int e = (int)blockIdx.x * (int)blockDim.x + (int)threadIdx.x; e < nin; e += ctas * (int)blockDim.x) {
+        const int c = L.clist[e];
+        float off = 0.0f;
+        if (!ZS) {
+            const unsigned cc = L.ccode[c];
+            const int step[6] = {-1, 1, -n1, n1, -n1 * n2, n1 * n2};
+            float v[6];
+#pragma unroll
+            for (int d = 0; d < 6; d++) v[d] = (cc & (1u << d)) ? src.coarse(c + step[d]) : 0.0f;
+#pragma unroll
+            for (int d = 0; d < 6; d++)
+                if (cc & (1u << d)) off += COARSE_COARSE * v[d];
+        }
+        f((int64_t)c, off);
+    }
+}
 
 // ---- coefficients, level 0 (src/sflip.jl:1315-1451) ----
 // finecoef_kernel! (:1324-1333), the three axes (blockIdx.y)
@@ -389,12 +480,12 @@ __global__ void __launch_bounds__(SPT) k_sp_coarsecoef(Topo t, float* cu, float*
 // active (not SOLID), bit 13 LIQUID) and its whole diagonal dg0 = dD + the positive
 // couplings, added in finerow's order (the same Float32 sums finerow forms every sweep); the
 // coarse part marks the coarse unknowns (LIQUID, no fine block over them) for the dots.
-__device__ __forceinline__ unsigned ccode(float c) { return c == FINE_FINE ? 2u : (c == FINE_COARSE ? 1u : 0u); }
+__device__ __forceinline__ unsigned coupling_code(float c) { return c == FINE_FINE ? 2u : (c == FINE_COARSE ? 1u : 0u); }
 __global__ void __launch_bounds__(SPT) k_sp_dirichlet(Topo t, float* dDf, float* dDc, uint8_t* actc, const uint8_t* tf,
                                                       const uint8_t* tc, const float* phif, const float* phic,
                                                       const float* cfx, const float* cfy, const float* cfz,
                                                       uint16_t* code0, float* dg0, uint8_t* cmask, int* clist,
-                                                      int* nclist, int gf) {
+                                                      int* nclist, uint8_t* ccode, int gf) {
     pdl_wait();
     pdl_trigger();
     if (sp_is_fine(gf)) {
@@ -427,7 +518,7 @@ __global__ void __launch_bounds__(SPT) k_sp_dirichlet(Topo t, float* dDf, float*
 #pragma unroll
             for (int m = 0; m < 6; m++) {
                 if (c6[m] > 0.0f) dg += c6[m];
-                code |= ccode(c6[m]) << (2 * m);
+                code |= coupling_code(c6[m]) << (2 * m);
             }
             code0[n] = (uint16_t)code;
             dg0[n] = dg;
@@ -440,6 +531,8 @@ __global__ void __launch_bounds__(SPT) k_sp_dirichlet(Topo t, float* dDf, float*
             coarse_cell(t, c, I, J, K);
             const bool cov = covered(t, I, J, K);
             float d = 0.0f;
+            bool edge = false;   // beside a fine block
+            unsigned cc = 0;
             if (tc[c] == LIQUID && !cov) {
                 const float pc = phic[c];
                 for (int a = 1; a <= 3; a++) {
@@ -448,6 +541,7 @@ __global__ void __launch_bounds__(SPT) k_sp_dirichlet(Topo t, float* dDf, float*
                         const int In = I + sg * e0, Jn = J + sg * e1, Kn = K + sg * e2;
                         if (!(0 <= In && In < n1 && 0 <= Jn && Jn < n2 && 0 <= Kn && Kn < n3)) continue;
                         if (covered(t, In, Jn, Kn)) {
+                            edge = true;
                             for (int q = 0; q < 4; q++)
                                 for (int p = 0; p < 4; p++) {
                                     const int FI = a == 1 ? (sg > 0 ? RATIO * In : RATIO * I - 1) : RATIO * I + p;
@@ -458,6 +552,8 @@ __global__ void __launch_bounds__(SPT) k_sp_dirichlet(Topo t, float* dDf, float*
                                 }
                         } else if (tc[lin(t.nc, In, Jn, Kn)] == AIR) {
                             d += COARSE_COARSE / theta<float>(pc, phic[lin(t.nc, In, Jn, Kn)]);
+                        } else if (tc[lin(t.nc, In, Jn, Kn)] == LIQUID) {
+                            cc |= 1u << (2 * (a - 1) + (sg > 0 ? 1 : 0));
                         }
                     }
                 }
@@ -465,7 +561,9 @@ __global__ void __launch_bounds__(SPT) k_sp_dirichlet(Topo t, float* dDf, float*
             dDc[c] = d;
             actc[c] = (tc[c] == LIQUID && !cov) ? 1 : 0;
             cmask[c] = actc[c];
-            if (actc[c]) clist[atomicAdd(nclist, 1)] = (int)c;
+            ccode[c] = (uint8_t)cc;
+            if (actc[c] && !edge) clist[atomicAdd(nclist, 1)] = (int)c;
+            if (actc[c] && edge) clist[(int)nc - 1 - atomicAdd(nclist + 1, 1)] = (int)c;
         }
     }
 }
@@ -1139,17 +1237,13 @@ __global__ void __launch_bounds__(T8) k_sp_blk8(Topo t, Comp L, const float* dg1
         }
         *reinterpret_cast<float4*>(outf + n) = make_float4(out[0], out[1], out[2], out[3]);
     } else {
-        SP_ACTIVE_LOOP(c, L, gf) {
-            int I, J, K;
-            coarse_cell(t, c, I, J, K);
-            float diag, off;
-            coarserow<8, ZS>(t, L, xf, xc, I, J, K, diag, off);
-            const float x0 = ZS ? 0.0f : xc[c];
+        coarse_rows<8, ZS>(t, L, SrcX{xf, xc}, gf, [&](int64_t c, float off) {
+            const float x0 = ZS ? 0.0f : xc[c], diag = L.dgc[c];
             float v;
             if (OP == BOP_RES) v = bc[c] - (diag * x0 - off);
             else v = diag > 0.0f ? x0 + OMEGA * (bc[c] - (diag * x0 - off)) / diag : 0.0f;
             outc[c] = v;
-        }
+        });
     }
 }
 
