@@ -166,6 +166,10 @@ __global__ void __launch_bounds__(SPT) k_sp_rhs(Topo t, const uint8_t* tf, const
 #define SP_SLOT_PIECES(n)                                                                   \
     for (int m_ = 0; m_ < 4; m_++)                                                          \
         if (const int64_t n = (int64_t)(sl - 1) * BCELLS + 4 * ((int)threadIdx.x + 256 * m_); true)
+// the same, of the pieces that hold a LIQUID cell
+#define SP_LIQUID_PIECES(n, words)                                                          \
+    _Pragma("unroll") for (int m_ = 0; m_ < 4; m_++)                                         \
+        if (const int64_t n = (int64_t)(sl - 1) * BCELLS + 4 * ((int)threadIdx.x + 256 * m_); piece_of(words, m_))
 // the slots of a fine part of gf CTAs, each CTA every gf-th from its own
 #define SP_SLOTS(sl, gf) for (int sl = sp_slot(gf); sl <= t.nslots; sl += (gf))
 #define SP_COARSE_PIECES(c, nc4, gf)                                                        \
@@ -190,7 +194,8 @@ __device__ __forceinline__ double dot4m(float4 a, float4 b, uchar4 m, uint8_t wa
 // prolongation from level 1, fused with it.
 template <int OP, class Src>
 __global__ void __launch_bounds__(SPT, 6) k_sp_blk(Topo t, Comp L, const uint16_t* code0, const float* dg0, float* outf,
-                                                float* outc, Src src, const float* bf, const float* bc, int gf) {
+                                                float* outc, Src src, const float* bf, const float* bc,
+                                                const uint32_t* pm, int pstride, int gf) {
     __shared__ float xs[PCELLS];
     pdl_wait();
     pdl_trigger();
@@ -198,12 +203,13 @@ __global__ void __launch_bounds__(SPT, 6) k_sp_blk(Topo t, Comp L, const uint16_
         const int sl = sp_slot(gf);
         int w[3];
         where_of(t, sl, w);
-        if (w[0] < 0) return;
+        const uint32_t words = piece_words(pm, pstride, sl);
+        if (w[0] < 0 || !__any_sync(0xffffffffu, words != 0u)) return;  // (every warp alike)
         if (OP != BOP_JAC_ZS) {
-            stage_block_s(t, src, sl, w, xs);
+            stage_block_s(t, src, sl, w, words, xs);
             __syncthreads();
         }
-        block_cells<OP>(code0, dg0, bf, xs, sl, [&](int64_t n, const float* v, const float*) {
+        block_cells<OP>(code0, dg0, bf, xs, sl, words, [&](int64_t n, const float* v, const float*) {
             st4(outf + n, make_float4(v[0], v[1], v[2], v[3]));
         });
     } else {
@@ -238,10 +244,11 @@ __global__ void __launch_bounds__(SPT) k_sp_dgc(Topo t, Comp L, float* dgc) {
 // slot sl through the staged block; `sink(n, q[4], x[4])`.
 template <class Sink>
 __device__ __forceinline__ void apply_block(const Topo& t, const uint16_t* code0, const float* dg0, const float* xf,
-                                            const float* xc, int sl, const int w[3], float* xs, Sink&& sink) {
-    stage_block(t, xf, xc, sl, w, xs);
+                                            const float* xc, int sl, const int w[3], uint32_t words, float* xs,
+                                            Sink&& sink) {
+    stage_block(t, xf, xc, sl, w, words, xs);
     __syncthreads();
-    block_cells<BOP_APPLY>(code0, dg0, nullptr, xs, sl, sink);
+    block_cells<BOP_APPLY>(code0, dg0, nullptr, xs, sl, words, sink);
 }
 
 // r = b - A P (apply! then xpby!(r, b, -1)), |b| and |r| (src/sflip.jl:1870-1877).
@@ -258,7 +265,7 @@ __global__ void __launch_bounds__(SPT) k_sp_start(Topo t, Comp L, const uint16_t
         int w[3];
         where_of(t, sl, w);
         if (w[0] >= 0)
-            apply_block(t, code0, dg0, Pf, Pc, sl, w, xs, [&](int64_t n, const float* q, const float*) {
+            apply_block(t, code0, dg0, Pf, Pc, sl, w, ~0u, xs, [&](int64_t n, const float* q, const float*) {
                 const float4 b = ld4(bf + n);
                 const float4 r = make_float4(b.x + (-1.0f) * q[0], b.y + (-1.0f) * q[1], b.z + (-1.0f) * q[2],
                                              b.w + (-1.0f) * q[3]);
@@ -342,7 +349,7 @@ __global__ void __launch_bounds__(SPT) k_sp_dinit(Topo t, const uint8_t* tf, con
 __global__ void __launch_bounds__(SPT, 6) k_sp_apply_dot(Topo t, Comp L, const uint16_t* code0, const float* dg0,
                                                       const uint8_t* tf, const uint8_t* cmask, const float* df,
                                                       const float* dc, float* qf, float* qc, SpState* st,
-                                                      double* partials, unsigned* counter, int gf) {
+                                                      double* partials, unsigned* counter, const uint32_t* pm, int gf) {
     __shared__ float xs[PCELLS];
     pdl_wait();
     pdl_trigger();
@@ -352,8 +359,9 @@ __global__ void __launch_bounds__(SPT, 6) k_sp_apply_dot(Topo t, Comp L, const u
         const int sl = sp_slot(gf);
         int w[3];
         where_of(t, sl, w);
-        if (w[0] >= 0)
-            apply_block(t, code0, dg0, df, dc, sl, w, xs, [&](int64_t n, const float* q, const float* x) {
+        const uint32_t words = piece_words(pm, 32, sl);
+        if (w[0] >= 0 && __any_sync(0xffffffffu, words != 0u))
+            apply_block(t, code0, dg0, df, dc, sl, w, words, xs, [&](int64_t n, const float* q, const float* x) {
                 st4(qf + n, make_float4(q[0], q[1], q[2], q[3]));
                 acc[0] += dot4m(make_float4(x[0], x[1], x[2], x[3]), make_float4(q[0], q[1], q[2], q[3]),
                                 ldm4(tf + n), LIQUID);
@@ -395,7 +403,7 @@ __device__ __forceinline__ float4 upd_piece(float* P, float* r, float* ro, const
 __global__ void __launch_bounds__(SPT) k_sp_update(Topo t, const uint8_t* tf, const uint8_t* cmask, float* Pf, float* Pc,
                                                    float* rf, float* rc, float* rof, float* roc, const float* df,
                                                    const float* dc, const float* qf, const float* qc, SpState* st,
-                                                   double* partials, unsigned* counter, int gf,
+                                                   double* partials, unsigned* counter, const uint32_t* pm, int gf,
                                                    cudaGraphConditionalHandle cond, int use_cond) {
     pdl_wait();
     pdl_trigger();
@@ -406,10 +414,13 @@ __global__ void __launch_bounds__(SPT) k_sp_update(Topo t, const uint8_t* tf, co
     const float alpha = st->alpha, ma = -alpha;
     double acc[1] = {0.0};
     if (sp_is_fine(gf)) {
-        SP_SLOTS(sl, gf) if (slot_used(t, sl)) SP_SLOT_PIECES(n) {
+        SP_SLOTS(sl, gf) {
+            const uint32_t words = piece_words(pm, 32, sl);
+            SP_LIQUID_PIECES(n, words) {
                 const float4 r = upd_piece(Pf + n, rf + n, rof + n, df + n, qf + n, alpha, ma);
                 acc[0] += dot4m(r, r, ldm4(tf + n), LIQUID);
             }
+        }
     } else {
         SP_COARSE_PIECES(c, (int64_t)t.nc[0] * t.nc[1] * t.nc[2] / 4, gf) {
             const float4 r = upd_piece(Pc + c, rc + c, roc + c, dc + c, qc + c, alpha, ma);
@@ -434,18 +445,21 @@ __global__ void __launch_bounds__(SPT) k_sp_update(Topo t, const uint8_t* tf, co
 __global__ void __launch_bounds__(SPT) k_sp_dot2(Topo t, const uint8_t* tf, const uint8_t* cmask, const float* zf,
                                                  const float* zc, const float* rf, const float* rc, const float* rof,
                                                  const float* roc, SpState* st, double* partials, unsigned* counter,
-                                                 int gf) {
+                                                 const uint32_t* pm, int gf) {
     pdl_wait();
     pdl_trigger();
     if (st->done) return;
     double acc[2] = {0.0, 0.0};
     if (sp_is_fine(gf)) {
-        SP_SLOTS(sl, gf) if (slot_used(t, sl)) SP_SLOT_PIECES(n) {
+        SP_SLOTS(sl, gf) {
+            const uint32_t words = piece_words(pm, 32, sl);
+            SP_LIQUID_PIECES(n, words) {
                 const float4 z = ld4(zf + n);
                 const uchar4 m = ldm4(tf + n);
                 acc[0] += dot4m(z, ld4(rf + n), m, LIQUID);
                 acc[1] += dot4m(z, ld4(rof + n), m, LIQUID);
             }
+        }
     } else {
         SP_COARSE_PIECES(c, (int64_t)t.nc[0] * t.nc[1] * t.nc[2] / 4, gf) {
             const float4 z = ld4(zc + c);
@@ -474,7 +488,7 @@ __global__ void __launch_bounds__(SPT) k_sp_dot2(Topo t, const uint8_t* tf, cons
 
 // d = z + beta d (xpby!, src/sflip.jl:1902).
 __global__ void __launch_bounds__(SPT) k_sp_xpby(Topo t, float* df, float* dc, const float* zf, const float* zc,
-                                                 const SpState* st, int gf) {
+                                                 const SpState* st, const uint32_t* pm, int gf) {
     pdl_wait();
     pdl_trigger();
     if (st->done) return;
@@ -484,7 +498,10 @@ __global__ void __launch_bounds__(SPT) k_sp_xpby(Topo t, float* df, float* dc, c
         st4(d, make_float4(zz.x + beta * dd.x, zz.y + beta * dd.y, zz.z + beta * dd.z, zz.w + beta * dd.w));
     };
     if (sp_is_fine(gf)) {
-        SP_SLOTS(sl, gf) if (slot_used(t, sl)) SP_SLOT_PIECES(n) piece(df + n, zf + n);
+        SP_SLOTS(sl, gf) {
+            const uint32_t words = piece_words(pm, 32, sl);
+            SP_LIQUID_PIECES(n, words) piece(df + n, zf + n);
+        }
     } else {
         SP_COARSE_PIECES(c, (int64_t)t.nc[0] * t.nc[1] * t.nc[2] / 4, gf) piece(dc + c, zc + c);
     }
@@ -535,7 +552,7 @@ __global__ void __launch_bounds__(SPT) k_sp_apply(Topo t, Comp L, const uint16_t
         int w[3];
         where_of(t, sl, w);
         if (w[0] < 0) return;
-        apply_block(t, code0, dg0, xf, xc, sl, w, xs, [&](int64_t n, const float* q, const float*) {
+        apply_block(t, code0, dg0, xf, xc, sl, w, ~0u, xs, [&](int64_t n, const float* q, const float*) {
             st4(qf + n, make_float4(q[0], q[1], q[2], q[3]));
         });
     } else {
@@ -699,6 +716,7 @@ struct mpp_sparse_ctx {
     float *cf[3], *cc[3], *dDf, *dDc;
     uint16_t* code0;    // each fine cell's six couplings, active and LIQUID bits (the block kernels)
     float* dg0;         // each fine cell's whole diagonal
+    uint32_t *pm, *pm_all;  // each slot's pieces that hold a LIQUID cell (1024 bits), and a slot's all
     uint8_t* cmask;     // the coarse unknowns (LIQUID, no fine block over them)
     uint8_t* ccode;     // which of their coarse neighbours couple
     float *dgc, *dgc1;  // and their whole diagonals at levels 0 and 1
@@ -834,6 +852,11 @@ struct SpRun {
     mpp_sparse_ctx* c;
     cudaStream_t s;
     int64_t nk = 0;
+    // whether the V-cycle takes every piece: its input may be nonzero off the water (the V-cycle
+    // entry's is the caller's), or its output array is not one that the operator clears there
+    bool all_pieces = false;
+    const uint32_t* pm() const { return all_pieces ? c->pm_all : c->pm; }
+    int ps() const { return all_pieces ? 0 : 32; }
 
     int grid1(int64_t n) const { return cap_blocks(c, n); }
 
@@ -851,7 +874,7 @@ struct SpRun {
             cudaMemsetAsync(a, 0, sizeof(float) * (size_t)c->ncc, s);
         sp_launch(k_sp_dirichlet, dim3(sp.g), SPT, s, t, c->dDf, c->dDc, c->actc, b->types_f, b->types_c, b->phi_f,
                   b->phi_c, (const float*)c->cf[0], (const float*)c->cf[1], (const float*)c->cf[2], c->code0, c->dg0,
-                  c->cmask, c->clist, c->nclist, c->ccode, sp.gf);
+                  c->cmask, c->clist, c->nclist, c->ccode, (uint8_t*)c->pm, c->zf, c->tmf, c->res0f, sp.gf);
         sp_launch(k_sp_dgc<16>, dim3(cap_blocks(c, c->ncc)), SPT, s, t, comp0(c, b->types_f), c->dgc);
         nk += 4;
         hierarchy(b->types_f);
@@ -894,18 +917,18 @@ struct SpRun {
                 if (q == 0 && from_zero) {
                     const SrcZS z{code0, dg0, bf, c->cmask, c->dgc, bc};
                     sp_launch(k_sp_blk<BOP_JAC, SrcZS>, dim3(sp.g), SPT, s, c->t, L, code0, dg0, xf, xc, z, bf, bc,
-                              sp.gf);
+                              pm(), ps(), sp.gf);
                     nk++;
                     continue;
                 }
                 if (q == 0 && pro)
                     sp_launch(k_sp_blk<BOP_JAC, SrcPro>, dim3(sp.g), SPT, s, c->t, L, code0, dg0, tf_, tc_, *pro, bf,
-                              bc, sp.gf);
+                              bc, pm(), ps(), sp.gf);
                 else
                     sp_launch(k_sp_blk<BOP_JAC, SrcX>, dim3(sp.g), SPT, s, c->t, L, code0, dg0, tf_, tc_,
-                              SrcX{xf, xc}, bf, bc, sp.gf);
+                              SrcX{xf, xc}, bf, bc, pm(), ps(), sp.gf);
                 sp_launch(k_sp_blk<BOP_JAC, SrcX>, dim3(sp.g), SPT, s, c->t, L, code0, dg0, xf, xc,
-                          SrcX{tf_, tc_}, bf, bc, sp.gf);
+                          SrcX{tf_, tc_}, bf, bc, pm(), ps(), sp.gf);
                 nk += 2;
             }
             return;
@@ -942,7 +965,8 @@ struct SpRun {
         smooth<16>(L0, zf, zc, rf, rc, c->tmf, c->tmc, sweeps, true);
         const Split sb = split_blk(c);
         sp_launch(k_sp_blk<BOP_RES, SrcX>, dim3(sb.g), SPT, s, t, L0, (const uint16_t*)c->code0,
-                  (const float*)c->dg0, c->res0f, c->res0c, SrcX{zf, zc}, rf, rc, sb.gf);
+                  (const float*)c->dg0, c->res0f, c->res0c, SrcX{zf, zc}, rf, rc,
+                  pm(), ps(), sb.gf);
         sp_launch(k_sp_restrict01, dim3(grid1((int64_t)t.nslots * BCELLS1)), SPT, s, t, c->b1f,
                   (const float*)c->res0f);
         nk += 2;
@@ -1006,11 +1030,11 @@ struct SpRun {
         const Split s0 = split_blk(c);
         sp_launch(k_sp_apply_dot, dim3(s0.g), SPT, s, t, L0, (const uint16_t*)c->code0, (const float*)c->dg0,
                   b->types_f, (const uint8_t*)c->cmask, (const float*)c->df, (const float*)c->dc, c->qf, c->qc, c->st,
-                  c->partials, c->counters + SCNT_DQ, s0.gf);
+                  c->partials, c->counters + SCNT_DQ, (const uint32_t*)c->pm, s0.gf);
         const Split sv = split_vec(c);
         sp_launch(k_sp_update, dim3(sv.g), SPT, s, t, b->types_f, (const uint8_t*)c->cmask, b->P_f, b->P_c, c->rf, c->rc, c->rof,
                   c->roc, (const float*)c->df, (const float*)c->dc, (const float*)c->qf, (const float*)c->qc, c->st,
-                  c->partials, c->counters + SCNT_UPD, sv.gf, cond, use_cond);
+                  c->partials, c->counters + SCNT_UPD, (const uint32_t*)c->pm, sv.gf, cond, use_cond);
         nk += 2;
     }
     // the rotated loop body: the V-cycle of the new residual, beta, d, then q, alpha, the update
@@ -1020,9 +1044,9 @@ struct SpRun {
         vcycle(b->types_f, c->zf, c->zc, c->rf, c->rc, o->sweeps, o->coarse, o->boost);
         sp_launch(k_sp_dot2, dim3(sv.g), SPT, s, t, b->types_f, (const uint8_t*)c->cmask, (const float*)c->zf, (const float*)c->zc,
                   (const float*)c->rf, (const float*)c->rc, (const float*)c->rof, (const float*)c->roc, c->st,
-                  c->partials, c->counters + SCNT_DOT2, sv.gf);
+                  c->partials, c->counters + SCNT_DOT2, (const uint32_t*)c->pm, sv.gf);
         sp_launch(k_sp_xpby, dim3(sv.g), SPT, s, t, c->df, c->dc, (const float*)c->zf, (const float*)c->zc,
-                  (const SpState*)c->st, sv.gf);
+                  (const SpState*)c->st, (const uint32_t*)c->pm, sv.gf);
         nk += 2;
         cg_step(b, cond, use_cond);
     }
@@ -1099,6 +1123,7 @@ int fgmres(mpp_sparse_ctx* c, SpRun& run, const mpp_sparse_basin* b, const mpp_s
         c->fg_alloc = true;
     }
     const uint8_t *tf = b->types_f, *tc = b->types_c;
+    run.all_pieces = true;
     *its = 0;
     *status = MPP_OK;
     *rel = 0.0f;
@@ -1133,7 +1158,7 @@ int fgmres(mpp_sparse_ctx* c, SpRun& run, const mpp_sparse_basin* b, const mpp_s
             const Split s0 = split_blk(c);
             sp_launch(k_sp_blk<BOP_JAC_ZS, SrcX>, dim3(s0.g), SPT, run.s, c->t, comp0(c, tf),
                       (const uint16_t*)c->code0, (const float*)c->dg0, c->Zf[j], c->Zc[j],
-                      SrcX{nullptr, nullptr}, (const float*)c->Vf[j], (const float*)c->Vc[j], s0.gf);
+                      SrcX{nullptr, nullptr}, (const float*)c->Vf[j], (const float*)c->Vc[j], (const uint32_t*)c->pm_all, 0, s0.gf);
             run.nk++;
             axpy(c, run, c->Zf[j], c->Zc[j], 1.0f, c->zf, c->zc, 0, 0);
             apply_(c, run, tf, c->Zf[j], c->Zc[j], c->qf, c->qc);
@@ -1391,6 +1416,9 @@ int mpp_sparse_ctx_create(mpp_sparse_ctx** out, const mpp_sparse_grid* g, int32_
     if (!e) e = sp_alloc_n(c, &c->dg0, nf);
     if (!e) e = sp_alloc_n(c, &c->cmask, c->ncc);
     if (!e) e = sp_alloc_n(c, &c->clist, c->ncc);
+    if (!e) e = sp_alloc_n(c, &c->pm, (int64_t)c->capacity * 32);
+    if (!e) e = sp_alloc_n(c, &c->pm_all, 32);
+    if (!e && cudaMemset(c->pm_all, 0xff, 32 * sizeof(uint32_t)) != cudaSuccess) e = MPP_ERR_CUDA;
     if (!e) e = sp_alloc_n(c, &c->nclist, 2);
     if (!e) e = sp_alloc_n(c, &c->ccode, c->ncc);
     if (!e) e = sp_alloc_n(c, &c->dgc1, c->ncc);
@@ -1505,6 +1533,7 @@ int mpp_sparse_vcycle(mpp_sparse_ctx* c, const mpp_sparse_basin* b, const float*
     }
     SpRun run{c, (cudaStream_t)stream};
     SCK(cudaMemsetAsync(zc, 0, sizeof(float) * (size_t)c->ncc, run.s));  // as mpp_sparse_apply's q
+    run.all_pieces = true;
     run.vcycle(b->types_f, zf, zc, rf, rc, sweeps, coarse, boost);
     return finish(c, run, nullptr, MPP_OK);
 }
