@@ -184,6 +184,7 @@ struct mpp_ctx {
     double* adv_acc[3];  // FP64 accumulators of the advection adjoint (face shapes), on first use
     // trapped-air fill (mpp_filltrapped), on first use: AIR and reached bit masks, the round
     // loop's state, and the graph of the round loop (a conditional WHILE node)
+    Walls walls;  // the walls as ranges, for the level-set passes
     uint32_t *trap_air, *trap_reach;
     TrapState* trap_st;
     cudaGraph_t trap_graph;
@@ -1426,6 +1427,89 @@ bool encode_level(CUtensorMap* m, CUtensorMapDataType dt, void* base, size_t es,
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The open (not SOLID) cells of each row (j, any k above the floor), Walls::rows: issolidcell's
+// px px + py py > R^2 holds for a prefix and a suffix of a row (px rises along it and rounding keeps
+// order), its pz < floor for the planes below some k, so ranges are its Float32 answers exactly.
+int build_walls(mpp_ctx* c) {
+    const mpp_grid& g = c->grid;
+    const float R2 = g.radius * g.radius;
+    std::vector<int2> rows((size_t)g.n[1] + 1);
+    for (int j = 0; j < g.n[1]; j++) {
+        const float py = g.lo[1] + ((float)j + 0.5f) * g.dx, pyy = py * py;
+        auto px = [&](int i) { return g.lo[0] + ((float)i + 0.5f) * g.dx; };
+        auto solid = [&](int i) { return px(i) * px(i) + pyy > R2; };
+        int a = 0, b = g.n[0];  // the first cell right of the axis, and from it the one nearest to it
+        while (a < b) {
+            const int m = (a + b) / 2;
+            if (px(m) < 0.f) a = m + 1;
+            else b = m;
+        }
+        int mid = a < g.n[0] ? a : g.n[0] - 1;
+        if (mid > 0 && solid(mid)) mid--;
+        int2 r = make_int2(0x7fffffff, -1);
+        if (!solid(mid)) {
+            int lo = 0, hi = mid;  // the first open cell
+            while (lo < hi) {
+                const int m = (lo + hi) / 2;
+                if (solid(m)) lo = m + 1;
+                else hi = m;
+            }
+            r.x = lo;
+            lo = mid;
+            hi = g.n[0] - 1;  // the last one
+            while (lo < hi) {
+                const int m = (lo + hi + 1) / 2;
+                if (solid(m)) hi = m - 1;
+                else lo = m;
+            }
+            r.y = lo;
+        }
+        rows[j] = r;
+    }
+    int lo = 0, hi = g.n[2];  // the first plane above the floor
+    while (lo < hi) {
+        const int m = (lo + hi) / 2;
+        if (g.lo[2] + ((float)m + 0.5f) * g.dx < g.floor_z) lo = m + 1;
+        else hi = m;
+    }
+    rows[g.n[1]] = make_int2(lo, 0);
+    // the quads' kinds, and the lists of those beside walls and of the open ones
+    std::vector<uint8_t> quad;
+    std::vector<uint32_t> list, clear;
+    const int rq = g.n[0] / 4;
+    if (g.n[0] % 4 == 0 && rq <= 65536 && g.n[1] <= 65536) {
+        const int2 none = make_int2(0x7fffffff, -1);
+        quad.resize((size_t)g.n[1] * rq);
+        for (int j = 0; j < g.n[1]; j++)
+            for (int q = 0; q < rq; q++) {
+                const int i = 4 * q;
+                const int2 r = rows[j], p = j + 1 < g.n[1] ? rows[j + 1] : none, m = j > 0 ? rows[j - 1] : none;
+                auto in = [](int2 a, int lo, int hi) { return lo >= a.x && hi <= a.y; };
+                auto out = [](int2 a, int lo, int hi) { return hi < a.x || lo > a.y; };
+                uint8_t kind = Walls::MIXED;
+                if (i > 0 && i + 4 < g.n[0] && in(r, i - 1, i + 4) && in(p, i, i + 3) && in(m, i, i + 3)) kind = Walls::CLEAR;
+                else if (out(r, i - 1, i + 4) && out(p, i, i + 3) && out(m, i, i + 3)) kind = Walls::SHUT;
+                quad[(size_t)j * rq + q] = kind;
+                if (kind != Walls::SHUT) (kind == Walls::CLEAR ? clear : list).push_back((uint32_t)j << 16 | (uint32_t)q);
+            }
+    }
+    c->walls.nlist = (int)list.size();
+    c->walls.nclear = (int)clear.size();
+    list.insert(list.end(), clear.begin(), clear.end());
+    auto put = [&](auto** to, const auto& v) -> int {
+        using T = typename std::remove_reference<decltype(v[0])>::type;
+        typename std::remove_const<T>::type* d = nullptr;
+        if (int e = alloc(c, (void**)&d, sizeof(T) * v.size())) return e;
+        if (!v.empty()) CK(cudaMemcpy(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
+        *to = d;
+        return MPP_OK;
+    };
+    if (int e = put(&c->walls.rows, rows)) return e;
+    if (int e = put(&c->walls.quad, quad)) return e;
+    if (int e = put(&c->walls.list, list)) return e;
+    return MPP_OK;
+}
+
 // The levels of k_cluster: from the first one of at most CL_CELLS cells whose planes (and those of
 // every smaller level) fit the shared memory of a cluster's CTAs, down to the coarsest. In the
 // environment MPP_CMG=0 keeps the per-level launches and MPP_CMG_MAXCELLS sets the size bound.
@@ -1714,6 +1798,7 @@ int mpp_ctx_create(mpp_ctx** out, const mpp_grid* g, const mpp_opts* o) {
     c->fg_residual = 0.0;
     c->vjp_beta = nullptr;
     for (int a = 0; a < 3; a++) c->adv_acc[a] = nullptr;
+    memset(&c->walls, 0, sizeof(c->walls));
     c->trap_air = c->trap_reach = nullptr;
     c->trap_st = nullptr;
     c->trap_graph = nullptr;
@@ -1858,6 +1943,7 @@ int mpp_ctx_create(mpp_ctx** out, const mpp_grid* g, const mpp_opts* o) {
         c->lv[0].dg = c->diag;
         c->lv[0].b = c->r;
     }
+    if ((e = build_walls(c))) return fail(e);
     if ((e = build_tma(c))) return fail(e);
     if ((e = build_cmg(c))) return fail(e);
     if (c->prec == MPP_PREC_FP64 && (e = alloc(c, &c->Pd, sizeof(double) * N))) return fail(e);
@@ -2553,9 +2639,18 @@ int mpp_extrapolate(mpp_ctx* c, float* u, float* v, float* w, uint8_t* fu, uint8
     }
     // a warp a word for the flags in and out, a thread a word for the layers
     const dim3 gwarp(grid_cells(c, 32 * ((words_max + EXT_WW - 1) / EXT_WW)), 3), gword(grid_cells(c, words_max), 3);
-    launch(k_extrap_flags, gwarp, TPB, 0, s, E);
+    bool f4 = true, x16 = true;  // the flags' and the faces' alignment
+    for (int a = 0; a < 3; a++) {
+        f4 = f4 && (reinterpret_cast<uintptr_t>(Fl[a]) & 3) == 0;
+        x16 = x16 && (reinterpret_cast<uintptr_t>(X[a]) & 15) == 0;
+    }
+    if (f4) launch(k_extrap_flags4, gword, TPB, 0, s, E);
+    else launch(k_extrap_flags, gwarp, TPB, 0, s, E);
     for (int l = 1; l <= layers; l++) launch(k_extrap_layer, gword, TPB, 0, s, E, l & 1);
-    launch(k_extrap_final, gwarp, TPB, 0, s, E, layers % 2 == 0 ? 1 : 0, layers == 0 ? 1 : 0);
+    const int in_a = layers % 2 == 0 ? 1 : 0, keep = layers == 0 ? 1 : 0;
+    const int64_t nmax = std::max(n[0], std::max(n[1], n[2]));
+    if (f4 && x16) launch(k_extrap_final4, dim3(grid_cells(c, (nmax + 3) / 4), 3), TPB, 0, s, E, in_a, keep);
+    else launch(k_extrap_final, gwarp, TPB, 0, s, E, in_a, keep);
     c->launches += layers + 2;
     CK(cudaGetLastError());
     return MPP_OK;
@@ -2662,23 +2757,21 @@ int mpp_redistance(mpp_ctx* c, float* phi, float* phi0, int iterations, uint8_t*
     cudaStream_t s = (cudaStream_t)stream;
     const Geo g = geo_of(c->grid);
     if (iterations == 0) {
-        if (types) {
-            launch(k_classify, grid_cells(c, N), TPB, 0, s, g, (const float*)phi, types);
-            c->launches++;
-        }
-        CK(cudaGetLastError());
-        return MPP_OK;
+        return types ? mpp_classify(c, types, phi, stream) : MPP_OK;
     }
+    const Walls& wl = c->walls;
     // phimax = Float32((iterations + 1) * dx) (src/flip.jl:674)
     const float phimax = (float)(iterations + 1) * c->grid.dx;
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-    const bool v4 = c->grid.n[0] % 4 == 0 && al(phi) && al(phi0) && (!types || (reinterpret_cast<uintptr_t>(types) & 3) == 0);
+    // quads: rows of whole ones (below 2^16 a row, and rows), arrays that take 16-byte loads
+    const bool v4 = c->grid.n[0] % 4 == 0 && c->grid.n[0] / 4 <= 65536 && c->grid.n[1] <= 65536 && al(phi) && al(phi0) &&
+                    (!types || (reinterpret_cast<uintptr_t>(types) & 3) == 0);
     float* src = phi;
     float* dst = phi0;
     for (int it = 0; it < iterations; it++) {
         uint8_t* ty = it + 1 == iterations ? types : nullptr;
-        if (v4) launch(k_reinit<4>, grid_cells(c, N / 4), TPB, 0, s, g, (const float*)src, dst, phimax, ty);
-        else launch(k_reinit<1>, grid_cells(c, N), TPB, 0, s, g, (const float*)src, dst, phimax, ty);
+        if (v4) launch(k_reinit4, grid_cells(c, N / 4), TPB, 0, s, g, wl, (const float*)src, dst, phimax, ty);
+        else launch(k_reinit, grid_cells(c, N), TPB, 0, s, g, wl, (const float*)src, dst, phimax, ty);
         std::swap(src, dst);
     }
     c->launches += iterations;
@@ -2693,7 +2786,13 @@ int mpp_classify(mpp_ctx* c, uint8_t* types, const float* phi, mpp_stream stream
         return MPP_ERR_INVALID;
     }
     const int64_t N = (int64_t)c->grid.n[0] * c->grid.n[1] * c->grid.n[2];
-    launch(k_classify, grid_cells(c, N), TPB, 0, (cudaStream_t)stream, geo_of(c->grid), phi, types);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (c->grid.n[0] % 4 == 0 && N < ((int64_t)1 << 31) && (reinterpret_cast<uintptr_t>(phi) & 15) == 0 &&
+        (reinterpret_cast<uintptr_t>(types) & 3) == 0) {
+        launch(k_classify4, grid_cells(c, N / 4), TPB, 0, s, geo_of(c->grid), c->walls, phi, types);
+    } else {
+        launch(k_classify, grid_cells(c, N), TPB, 0, s, geo_of(c->grid), phi, types);
+    }
     c->launches++;
     CK(cudaGetLastError());
     return MPP_OK;

@@ -16,8 +16,7 @@
 // reference's bit for bit, and moves a bit a face (the masks, which stay in L2) plus the
 // values on the front. A last pass writes the 0/1 flags and zeroes what no layer reached
 // and every walled face. One launch a pass covers all three arrays (blockIdx.y is the
-// array); the flags are read and written a warp a mask word (32 faces of a row, coalesced),
-// a layer takes a thread a mask word.
+// array).
 #pragma once
 
 #include "mpp_base.cuh"
@@ -142,12 +141,53 @@ __global__ void __launch_bounds__(TPB) k_extrap_flags(ExtBits E) {
     }
 }
 
-// Layer `layer` (1-based): Rn = R | D, and the values of the faces D reaches. A thread a mask
-// word; a word on the front takes its faces eight at a time (their loads before their
-// stores). `from_a`: the layer reads ra and writes rb (else the other way round).
+// The same with flags 4-byte aligned: a thread a word, whose 32 flags lie in nine aligned words of
+// the array (a row of n1 + 1 flags starts anywhere), shifted into place and reduced to bits four at a
+// time: a quarter of the load requests and of the instructions of a lane a flag (256^3: 56 -> 16 us).
+__global__ void __launch_bounds__(TPB) k_extrap_flags4(ExtBits E) {
+    pdl_wait();
+    pdl_trigger();
+    const int ax = blockIdx.y;
+    const ExtArr A = ext_arr(E, ax);
+    const uint8_t* fin = pick3(ax, E.f[0], E.f[1], E.f[2]);
+    uint32_t* R = pick3(ax, E.ra[0], E.ra[1], E.ra[2]);
+    const unsigned total = (unsigned)A.a1 * (unsigned)A.a2 * (unsigned)A.a3;
+    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < A.nw; w += gridDim.x * blockDim.x) {
+        const unsigned r = w / (unsigned)A.W;
+        const int i0 = 32 * (int)(w - r * (unsigned)A.W), cnt = A.a1 - i0 < 32 ? A.a1 - i0 : 32;
+        const unsigned id = r * (unsigned)A.a1 + (unsigned)i0, sh = 8u * (id & 3u);
+        uint32_t m = 0;
+        if ((id & ~3u) + 36u <= total) {
+            const uint32_t* p = reinterpret_cast<const uint32_t*>(fin + (id & ~3u));
+            uint32_t v[9];
+#pragma unroll
+            for (int q = 0; q < 9; q++) v[q] = p[q];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const uint32_t b = __funnelshift_r(v[q], v[q + 1], sh);
+                m |= (((__vcmpne4(b, 0u) & 0x08040201u) * 0x01010101u) >> 24) << (4 * q);
+            }
+            if (cnt < 32) m &= (1u << cnt) - 1u;
+        } else {  // the array's last faces
+            for (int b = 0; b < cnt; b++)
+                if (fin[id + (unsigned)b] != 0) m |= 1u << b;
+        }
+        R[w] = m;
+    }
+}
+
+// Layer `layer` (1-based): Rn = R | D, and the values of the faces D reaches. A thread scans a mask
+// word; the words on the front are gathered in shared memory and shared out over the block's warps, a
+// lane a face (so a row's values are consecutive loads), LAYER_WW words a warp at a time. A warp's
+// words follow each other, the next words are another block's: a front, which is a sheet of words that
+// follow each other, meets every SM. (A thread that took its word's 32 faces alone: 18 us a layer at
+// 256^3, here 15.) `from_a`: the layer reads ra and writes rb (else the other way round).
+constexpr int LAYER_WW = 4;
 __global__ void __launch_bounds__(TPB) k_extrap_layer(ExtBits E, int from_a) {
     pdl_wait();
     pdl_trigger();
+    __shared__ uint32_t fw[TPB], fm[7][TPB];  // the front's words: index; D and the neighbours' validity
+    __shared__ int nfront;
     const int ax = blockIdx.y;
     const ExtArr A = ext_arr(E, ax);
     const uint32_t* R = from_a ? pick3(ax, E.ra[0], E.ra[1], E.ra[2]) : pick3(ax, E.rb[0], E.rb[1], E.rb[2]);
@@ -156,53 +196,68 @@ __global__ void __launch_bounds__(TPB) k_extrap_layer(ExtBits E, int from_a) {
     float* x = pick3(ax, E.x[0], E.x[1], E.x[2]);
     const unsigned PY = (unsigned)A.W, PZ = (unsigned)A.W * (unsigned)A.a2;
     const unsigned s1 = (unsigned)A.a1, s2 = (unsigned)A.a1 * (unsigned)A.a2;
-    for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < A.nw; w += gridDim.x * blockDim.x) {
-        const unsigned r = w / (unsigned)A.W;
-        const int wx = (int)(w % (unsigned)A.W);
-        const int j = (int)(r % (unsigned)A.a2), k = (int)(r / (unsigned)A.a2);
-        const uint32_t rc = R[w], o = O[w];
-        const uint32_t rl = wx > 0 ? R[w - 1] : 0u, rr = wx + 1 < A.W ? R[w + 1] : 0u;
-        const uint32_t ryp = j + 1 < A.a2 ? R[w + PY] : 0u, rym = j > 0 ? R[w - PY] : 0u;
-        const uint32_t rzp = k + 1 < A.a3 ? R[w + PZ] : 0u, rzm = k > 0 ? R[w - PZ] : 0u;
-        // neighbour validity, bit i of each: the face at +x, -x, +y, -y, +z, -z of face i
-        const uint32_t vxp = (rc >> 1) | (rr << 31), vxm = (rc << 1) | (rl >> 31);
-        uint32_t d = (vxp | vxm | ryp | rym | rzp | rzm) & o & ~rc;
-        Rn[w] = rc | d;
-        const unsigned base = r * s1 + 32u * (unsigned)wx;
-        while (d) {
-            int bits[8];
-            int nb = 0;
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                bits[q] = d ? __ffs(d) - 1 : -1;
-                if (d) {
-                    d &= d - 1;
-                    nb++;
-                }
+    const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
+    for (unsigned w0 = 0; w0 < A.nw; w0 += gridDim.x * blockDim.x) {
+        if (threadIdx.x == 0) nfront = 0;
+        __syncthreads();
+        const unsigned w = w0 + ((unsigned)warp * gridDim.x + blockIdx.x) * 32u + (unsigned)lane;
+        if (w < A.nw) {
+            const unsigned r = w / (unsigned)A.W;
+            const int wx = (int)(w - r * (unsigned)A.W);
+            const unsigned k = r / (unsigned)A.a2;
+            const int j = (int)(r - k * (unsigned)A.a2);
+            const uint32_t rc = R[w], o = O[w];
+            const uint32_t rl = wx > 0 ? R[w - 1] : 0u, rr = wx + 1 < A.W ? R[w + 1] : 0u;
+            const uint32_t ryp = j + 1 < A.a2 ? R[w + PY] : 0u, rym = j > 0 ? R[w - PY] : 0u;
+            const uint32_t rzp = (int)k + 1 < A.a3 ? R[w + PZ] : 0u, rzm = k > 0 ? R[w - PZ] : 0u;
+            // neighbour validity, bit i of each: the face at +x, -x, +y, -y, +z, -z of face i
+            const uint32_t vxp = (rc >> 1) | (rr << 31), vxm = (rc << 1) | (rl >> 31);
+            const uint32_t d = (vxp | vxm | ryp | rym | rzp | rzm) & o & ~rc;
+            Rn[w] = rc | d;
+            if (d) {
+                const int e = atomicAdd(&nfront, 1);
+                fw[e] = w;
+                fm[0][e] = vxp;
+                fm[1][e] = vxm;
+                fm[2][e] = ryp;
+                fm[3][e] = rym;
+                fm[4][e] = rzp;
+                fm[5][e] = rzm;
+                fm[6][e] = d;
             }
-            float sum[8];
-            int cnt[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                sum[q] = 0.f;
-                cnt[q] = 0;
-                if (q >= nb) continue;
-                const int bit = bits[q];
-                const unsigned id = base + (unsigned)bit;
-                const bool take[6] = {((vxp >> bit) & 1u) != 0, ((vxm >> bit) & 1u) != 0, ((ryp >> bit) & 1u) != 0,
-                                      ((rym >> bit) & 1u) != 0, ((rzp >> bit) & 1u) != 0, ((rzm >> bit) & 1u) != 0};
-                const unsigned nbi[6] = {id + 1, id - 1, id + s1, id - s1, id + s2, id - s2};
-#pragma unroll
-                for (int e = 0; e < 6; e++)
-                    if (take[e]) {
-                        sum[q] = __fadd_rn(sum[q], x[nbi[e]]);
-                        cnt[q]++;
-                    }
-            }
-#pragma unroll
-            for (int q = 0; q < 8; q++)
-                if (q < nb) x[base + (unsigned)bits[q]] = __fdiv_rn(sum[q], (float)cnt[q]);
         }
+        __syncthreads();
+        const int n = nfront;
+        for (int e0 = warp; e0 < n; e0 += LAYER_WW * (TPB / 32)) {
+            unsigned id[LAYER_WW];
+            float v[LAYER_WW][6];
+#pragma unroll
+            for (int q = 0; q < LAYER_WW; q++) {
+                const int e = e0 + q * (TPB / 32);
+                if (e >= n || !((fm[6][e] >> lane) & 1u)) continue;
+                const unsigned r = fw[e] / (unsigned)A.W;
+                id[q] = r * s1 + 32u * (fw[e] - r * (unsigned)A.W) + (unsigned)lane;
+                const unsigned nbi[6] = {id[q] + 1, id[q] - 1, id[q] + s1, id[q] - s1, id[q] + s2, id[q] - s2};
+#pragma unroll
+                for (int m = 0; m < 6; m++)
+                    if ((fm[m][e] >> lane) & 1u) v[q][m] = x[nbi[m]];
+            }
+#pragma unroll
+            for (int q = 0; q < LAYER_WW; q++) {
+                const int e = e0 + q * (TPB / 32);
+                if (e >= n || !((fm[6][e] >> lane) & 1u)) continue;
+                float sum = 0.f;
+                int cnt = 0;
+#pragma unroll
+                for (int m = 0; m < 6; m++)
+                    if ((fm[m][e] >> lane) & 1u) {
+                        sum = __fadd_rn(sum, v[q][m]);
+                        cnt++;
+                    }
+                x[id[q]] = __fdiv_rn(sum, (float)cnt);
+            }
+        }
+        __syncthreads();  // (the list is the next words')
     }
 }
 
@@ -241,6 +296,53 @@ __global__ void __launch_bounds__(TPB) k_extrap_final(ExtBits E, int in_a, int k
             // unreached_kernel!, then solidify! (a walled face is zero, reached or not)
             if (!reached || !open) x[id] = 0.f;
             if (!keep_flags) f[id] = reached ? 1 : 0;
+        }
+    }
+}
+
+// Bits i .. i + 31 of row r of a mask (W words a row).
+__device__ __forceinline__ uint32_t row_bits(const uint32_t* M, unsigned r, int W, int i) {
+    const int w = i >> 5;
+    const uint32_t* p = M + (size_t)r * W + w;
+    return __funnelshift_r(p[0], w + 1 < W ? p[1] : 0u, (unsigned)i & 31u);
+}
+// The same with x 16-byte and the flags 4-byte aligned: a thread takes four faces that follow each
+// other in memory (they may run into the next row), and neighbouring threads neighbouring ones, so a
+// warp's stores are whole lines. Bound: the bytes written. (256^3, 72 us a lane a face -> 55; 16
+// faces a thread, whose 16-byte stores lie 64 bytes apart, 61.)
+__global__ void __launch_bounds__(TPB) k_extrap_final4(ExtBits E, int in_a, int keep_flags) {
+    pdl_wait();
+    pdl_trigger();
+    const int ax = blockIdx.y;
+    const ExtArr A = ext_arr(E, ax);
+    const uint32_t* R = in_a ? pick3(ax, E.ra[0], E.ra[1], E.ra[2]) : pick3(ax, E.rb[0], E.rb[1], E.rb[2]);
+    const uint32_t* O = pick3(ax, E.open[0], E.open[1], E.open[2]);
+    float* x = pick3(ax, E.x[0], E.x[1], E.x[2]);
+    uint8_t* f = pick3(ax, E.f[0], E.f[1], E.f[2]);
+    const unsigned total = (unsigned)A.a1 * (unsigned)A.a2 * (unsigned)A.a3;
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; 4u * p < total; p += gridDim.x * blockDim.x) {
+        const unsigned id = 4u * p, cnt = total - id < 4u ? total - id : 4u, r = id / (unsigned)A.a1;
+        const int i = (int)(id - r * (unsigned)A.a1);
+        uint32_t reached = row_bits(R, r, A.W, i), open = row_bits(O, r, A.W, i);  // (bits past the row are zeros)
+        for (unsigned got = (unsigned)(A.a1 - i), n = r + 1; got < cnt; got += (unsigned)A.a1, n++) {
+            reached |= row_bits(R, n, A.W, 0) << got;
+            open |= row_bits(O, n, A.W, 0) << got;
+        }
+        const uint32_t zero = ~(reached & open) & 15u;  // unreached_kernel!, then solidify!
+        if (cnt == 4u) {
+            if (!keep_flags) *reinterpret_cast<uint32_t*>(f + id) = ((reached & 15u) * 0x00204081u) & 0x01010101u;
+            if (zero == 15u) {
+                *reinterpret_cast<float4*>(x + id) = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+#pragma unroll
+                for (int b = 0; b < 4; b++)
+                    if ((zero >> b) & 1u) x[id + b] = 0.f;
+            }
+        } else {
+            for (unsigned b = 0; b < cnt; b++) {
+                if ((zero >> b) & 1u) x[id + b] = 0.f;
+                if (!keep_flags) f[id + b] = (reached >> b) & 1u;
+            }
         }
     }
 }

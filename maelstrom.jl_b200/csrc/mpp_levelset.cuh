@@ -3,12 +3,16 @@
 // trapped-air fill), src/flip.jl:608-760.
 //
 // Redistancing: a thread takes 4 consecutive cells of a row (16-byte loads of the row and
-// of the rows at -+y and -+z, one element each side for -+x); the wall test of the cell
-// and of its neighbours is the Float32 geometry of issolidcell, with the squares of the
-// x positions formed once per thread and shared by the cells. The arithmetic is the
+// of the rows at -+y and -+z, one element each side for -+x). The arithmetic is the
 // reference's, in its order, with Julia's min/max (the sign of a zero counts) and clamp;
 // the library is built without FMA contraction, so every cell is bit-identical to the
 // reference's Float32 code. The last sweep also writes the cell classes (classify!).
+// A sweep is bound by its instructions, not by its 8 bytes a cell, so the common cells
+// take few: the wall test of issolidcell is a range of open cells a row (Walls), four
+// cells with no wall beside them take a minimum and a maximum of their neighbours each
+// (which decide whether the surface passes, and whether the distance is beyond phimax), and
+// only a cell near the surface goes through Godunov's update. 256^3, a sweep: 138 us with
+// the Float32 wall geometry of seven cells and Julia's min on every pair, 61 here.
 //
 // Trapped air: the reference reaches air from the grid's top layer by rounds of sweeps of
 // one thread per line along z, x and y, until a round reaches nothing (a host read per
@@ -24,6 +28,7 @@
 #pragma once
 
 #include "mpp_base.cuh"
+#include "mpp_coarsest.cuh"
 
 namespace mpp {
 
@@ -65,136 +70,255 @@ __device__ __forceinline__ float eikonal(float a, float b, float c, float h) {
     return d;
 }
 
-// reinit_kernel! (src/flip.jl:631-666), one Jacobi sweep out <- phi, W cells of a row per
-// thread (W = 4: n1 a multiple of 4 and 16-byte aligned arrays; else W = 1). When `types`
-// is given the sweep is redistance!'s last and classify_kernel! (src/flip.jl:682-686) runs
-// on its output.
-template <int W>
-__global__ void __launch_bounds__(TPB) k_reinit(Geo g, const float* __restrict__ phi, float* __restrict__ out,
+// eikonal for three numbers of the same sign (no NaN), where the hardware's min and max are Julia's;
+// the division by 3 as div_small rounds it.
+__device__ __forceinline__ float eikonal_ord(float a, float b, float c, float h) {
+    float t0 = fminf(a, b), t1 = fmaxf(a, b);
+    a = t0;
+    b = t1;
+    t0 = fminf(b, c);
+    t1 = fmaxf(b, c);
+    b = t0;
+    c = t1;
+    t0 = fminf(a, b);
+    t1 = fmaxf(a, b);
+    a = t0;
+    b = t1;
+    float d = a + h;
+    if (d > b) {
+        const float ab = a - b;
+        d = 0.5f * (a + b + sqrtf(fmaxf(2.0f * h * h - ab * ab, 0.0f)));
+        if (d > c) {
+            const float t = a + b + c;
+            d = div_small(t + sqrtf(fmaxf(t * t - 3.0f * (a * a + b * b + c * c - h * h), 0.0f)), 3.0f, 1.0f / 3.0f);
+        }
+    }
+    return d;
+}
+// The walls as ranges (the context's build_walls): row (j, k)'s open (not SOLID) cells are x from
+// rows[j].x to rows[j].y when k >= rows[n2].x, none below.
+struct Walls {
+    // a quad (cells 4 q .. 4 q + 3 of row j): open with all cells around it in the plane, inside the
+    // walls likewise, or neither
+    enum : uint8_t { CLEAR = 0, SHUT = 1, MIXED = 2 };
+    const int2* rows;
+    const uint8_t* quad;   // [n2][n1 / 4], when n1 is a multiple of 4
+    const uint32_t* list;  // j << 16 | q of the MIXED quads, then of the CLEAR ones
+    int nlist, nclear;
+    __device__ __forceinline__ bool open(int2 r, int i) const { return i >= r.x && i <= r.y; }
+};
+
+// min and max that hand a NaN on
+__device__ __forceinline__ float nmin(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float nmax(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// reinit_kernel!'s value of a cell from its neighbours f (+x, -x, +y, -y, +z, -z; ok: in range and not
+// SOLID) in any case: walls beside it, NaN.
+__device__ __forceinline__ float reinit_cell(float cm, const float (&f)[6], unsigned ok, bool solid, float phimax, float h,
+                                             float far) {
+    if (solid) {
+        // a wall cell takes the lowest value of the water next to it
+        float lowest = cm;
+        bool found = false;
+#pragma unroll
+        for (int e = 0; e < 6; e++)
+            if (ok & (1u << e)) {
+                lowest = found ? jmin(lowest, f[e]) : f[e];
+                found = true;
+            }
+        return found ? lowest : (cm > phimax ? phimax : (cm < -phimax ? -phimax : cm));
+    }
+    const bool inside = cm < 0.0f;
+    bool frozen = false;
+    float ax = phimax, ay = phimax, az = phimax;
+#pragma unroll
+    for (int e = 0; e < 6; e++)
+        if (ok & (1u << e)) {
+            if ((f[e] < 0.0f) != inside) frozen = true;
+            const float d = fabsf(f[e]);
+            if (e < 2) ax = jmin(ax, d);
+            else if (e < 4) ay = jmin(ay, d);
+            else az = jmin(az, d);
+        }
+    if (frozen) return cm;
+    const float d = (ax == phimax && ay == phimax && az == phimax) ? far : jmin(eikonal(ax, ay, az, h), phimax);
+    return inside ? -d : d;
+}
+// One cell of a sweep in any place.
+__device__ __forceinline__ float reinit_any(const Geo& g, const Walls& wl, const float* phi, int i, int j, int k, int kf,
+                                            float phimax, float far, bool& solid) {
+    const int n1 = g.n[0], n2 = g.n[1], n3 = g.n[2];
+    const int64_t sy = n1, sz = (int64_t)n1 * n2, idx = i + sy * j + sz * k;
+    const int2 r0 = wl.rows[j];
+    const bool in = wl.open(r0, i), up = k >= kf;
+    const unsigned ok = (up && i + 1 < n1 && wl.open(r0, i + 1) ? 1u : 0u) | (up && i > 0 && wl.open(r0, i - 1) ? 2u : 0u) |
+                        (up && j + 1 < n2 && wl.open(wl.rows[j + 1 < n2 ? j + 1 : j], i) ? 4u : 0u) |
+                        (up && j > 0 && wl.open(wl.rows[j > 0 ? j - 1 : j], i) ? 8u : 0u) |
+                        (in && k + 1 < n3 && k + 1 >= kf ? 16u : 0u) | (in && k > 0 && k - 1 >= kf ? 32u : 0u);
+    const float f[6] = {ok & 1u ? phi[idx + 1] : 0.f,  ok & 2u ? phi[idx - 1] : 0.f,  ok & 4u ? phi[idx + sy] : 0.f,
+                        ok & 8u ? phi[idx - sy] : 0.f, ok & 16u ? phi[idx + sz] : 0.f, ok & 32u ? phi[idx - sz] : 0.f};
+    solid = !(in && up);
+    return reinit_cell(phi[idx], f, ok, solid, phimax, g.dx, far);
+}
+
+// reinit_kernel! (src/flip.jl:631-666), one Jacobi sweep out <- phi, four cells of a row a thread
+// (n1 a multiple of 4, 16-byte aligned arrays), and classify! with it when `types` is given.
+// Almost every warp's 128 cells of a row cross a wall, and the four cells there would make the
+// other 31 threads wait for their longer way (113 M issued warp instructions a sweep at 256^3, 12
+// threads in one). So the first loop takes the quads that are open with all around them and those
+// inside the walls, told by a byte each (Walls::quad, the same for every plane), and the second
+// the quads beside walls (Walls::list) of every plane and the open ones of the planes at the floor
+// and the top, a cell a thread. A thread's next quad is stepped (dq, dj, dk), not divided out.
+__global__ void __launch_bounds__(TPB) k_reinit4(Geo g, Walls wl, const float* __restrict__ phi, float* __restrict__ out,
+                                                 float phimax, uint8_t* __restrict__ types) {
+    pdl_wait();
+    pdl_trigger();
+    const int n1 = g.n[0], n2 = g.n[1], n3 = g.n[2], rq = n1 / 4;
+    const float h = g.dx;
+    const unsigned sy = (unsigned)n1, sz = (unsigned)n1 * (unsigned)n2;
+    // far from the surface every neighbour distance is phimax: the same update for every such cell
+    const float far = jmin(eikonal(phimax, phimax, phimax, h), phimax);
+    const int kf = wl.rows[n2].x;
+    const unsigned step = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned t = t0;
+    int q = (int)(t % (unsigned)rq), j = (int)(t / (unsigned)rq % (unsigned)n2), k = (int)(t / (unsigned)rq / (unsigned)n2);
+    const int dq = (int)(step % (unsigned)rq), dj = (int)(step / (unsigned)rq % (unsigned)n2),
+              dk = (int)(step / (unsigned)rq / (unsigned)n2);
+    for (; k < n3; t += step) {
+        const uint8_t kind = wl.quad[j * rq + q];
+        const unsigned base = 4u * t;
+        const bool solid = kind == Walls::SHUT;
+        if (solid || (kind == Walls::CLEAR && k > kf && k + 1 < n3)) {
+            const float4 C = *reinterpret_cast<const float4*>(phi + base);
+            const float c[4] = {C.x, C.y, C.z, C.w};
+            float o[4];
+            if (solid) {
+#pragma unroll
+                for (int m = 0; m < 4; m++) o[m] = c[m] > phimax ? phimax : (c[m] < -phimax ? -phimax : c[m]);
+            } else {
+                const float4 YP = *reinterpret_cast<const float4*>(phi + base + sy);
+                const float4 YM = *reinterpret_cast<const float4*>(phi + base - sy);
+                const float4 ZP = *reinterpret_cast<const float4*>(phi + base + sz);
+                const float4 ZM = *reinterpret_cast<const float4*>(phi + base - sz);
+                const float xl = phi[base - 1], xr = phi[base + 4];
+                const float yp[4] = {YP.x, YP.y, YP.z, YP.w}, ym[4] = {YM.x, YM.y, YM.z, YM.w},
+                            zp[4] = {ZP.x, ZP.y, ZP.z, ZP.w}, zm[4] = {ZM.x, ZM.y, ZM.z, ZM.w};
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    const float f[6] = {m < 3 ? c[m < 3 ? m + 1 : 0] : xr, m > 0 ? c[m > 0 ? m - 1 : 0] : xl, yp[m], ym[m],
+                                        zp[m], zm[m]};
+                    const float mx = nmax(nmax(nmax(f[0], f[1]), nmax(f[2], f[3])), nmax(f[4], f[5]));
+                    const float mn = nmin(nmin(nmin(f[0], f[1]), nmin(f[2], f[3])), nmin(f[4], f[5]));
+                    const bool inside = c[m] < 0.0f;
+                    // the surface passes when a neighbour's side differs; else the nearest one's distance
+                    // is that of the largest (smallest) value
+                    const bool frozen = inside ? !(mx < 0.0f) : mn < 0.0f;
+                    const float near = inside ? -mx : mn;
+                    float v = inside ? -far : far;
+                    if (frozen) v = c[m];
+                    if (!frozen && !(near >= phimax)) {
+                        if (!(mx == mx)) {  // (a NaN neighbour: on no side, so an inside cell was frozen)
+                            v = reinit_cell(c[m], f, 63u, false, phimax, h, far);
+                        } else {
+                            const float d = fminf(eikonal_ord(fminf(phimax, fminf(fabsf(f[0]), fabsf(f[1]))),
+                                                              fminf(phimax, fminf(fabsf(f[2]), fabsf(f[3]))),
+                                                              fminf(phimax, fminf(fabsf(f[4]), fabsf(f[5]))), h), phimax);
+                            v = inside ? -d : d;
+                        }
+                    }
+                    o[m] = v;
+                }
+            }
+            *reinterpret_cast<float4*>(out + base) = make_float4(o[0], o[1], o[2], o[3]);
+            if (types) {
+                uint8_t ty[4];
+#pragma unroll
+                for (int m = 0; m < 4; m++) ty[m] = solid ? SOLID : (o[m] < 0.0f ? LIQUID : AIR);
+                *reinterpret_cast<uchar4*>(types + base) = make_uchar4(ty[0], ty[1], ty[2], ty[3]);
+            }
+        }
+        q += dq;
+        j += dj;
+        k += dk;
+        if (q >= rq) {
+            q -= rq;
+            j++;
+        }
+        if (j >= n2) {
+            j -= n2;
+            k++;
+        }
+    }
+    // the rest, a cell a thread: quads beside walls in every plane, then the open quads of the planes
+    // 0 .. kf and n3 - 1
+    const unsigned walled = 4u * (unsigned)wl.nlist, nclear = 4u * (unsigned)wl.nclear;
+    const unsigned low = (unsigned)(kf + 1 < n3 ? kf + 1 : n3), planes = low < (unsigned)n3 ? low + 1u : low;
+    const unsigned all = walled * (unsigned)n3, end = all + nclear * planes;
+    for (unsigned e = t0; e < end; e += step) {
+        const bool w = e < all;
+        const unsigned x = w ? e : e - all, m = w ? walled : nclear, p = x / m, c = x - p * m;
+        const uint32_t jq = (w ? wl.list : wl.list + wl.nlist)[c >> 2];
+        const int kk = w ? (int)p : (p < low ? (int)p : n3 - 1), jj = (int)(jq >> 16), i = 4 * (int)(jq & 0xffffu) + (int)(c & 3u);
+        const int64_t idx = i + (int64_t)n1 * (jj + (int64_t)n2 * kk);
+        bool solid;
+        const float v = reinit_any(g, wl, phi, i, jj, kk, kf, phimax, far, solid);
+        out[idx] = v;
+        if (types) types[idx] = solid ? SOLID : (v < 0.0f ? LIQUID : AIR);
+    }
+}
+
+// classify_kernel! (src/flip.jl:682-686), four cells a thread (as k_reinit4; types 4-byte aligned).
+__global__ void __launch_bounds__(TPB) k_classify4(Geo g, Walls wl, const float* __restrict__ phi, uint8_t* __restrict__ types) {
+    pdl_wait();
+    pdl_trigger();
+    const int n2 = g.n[1], n3 = g.n[2], rq = g.n[0] / 4, kf = wl.rows[n2].x;
+    const unsigned step = gridDim.x * blockDim.x;
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    int q = (int)(t % (unsigned)rq), j = (int)(t / (unsigned)rq % (unsigned)n2), k = (int)(t / (unsigned)rq / (unsigned)n2);
+    const int dq = (int)(step % (unsigned)rq), dj = (int)(step / (unsigned)rq % (unsigned)n2),
+              dk = (int)(step / (unsigned)rq / (unsigned)n2);
+    for (; k < n3; t += step) {
+        const float4 C = *reinterpret_cast<const float4*>(phi + 4u * t);
+        const int2 r = wl.rows[j];
+        const float c[4] = {C.x, C.y, C.z, C.w};
+        uint8_t ty[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) ty[m] = !(wl.open(r, 4 * q + m) && k >= kf) ? SOLID : (c[m] < 0.0f ? LIQUID : AIR);
+        *reinterpret_cast<uchar4*>(types + 4u * t) = make_uchar4(ty[0], ty[1], ty[2], ty[3]);
+        q += dq;
+        j += dj;
+        k += dk;
+        if (q >= rq) {
+            q -= rq;
+            j++;
+        }
+        if (j >= n2) {
+            j -= n2;
+            k++;
+        }
+    }
+}
+
+// One Jacobi sweep, a cell a thread, for rows or arrays that k_reinit4 does not take.
+__global__ void __launch_bounds__(TPB) k_reinit(Geo g, Walls wl, const float* __restrict__ phi, float* __restrict__ out,
                                                 float phimax, uint8_t* __restrict__ types) {
     pdl_wait();
     pdl_trigger();
-    const int n1 = g.n[0], n2 = g.n[1], n3 = g.n[2];
-    const unsigned rq = (unsigned)(n1 / W);
-    const unsigned total = rq * (unsigned)n2 * (unsigned)n3;  // the host checks the grid fits 32 bits
-    const float dx = g.dx, h = g.dx, R2 = g.radius * g.radius;
-    const unsigned sy = (unsigned)n1, sz = (unsigned)n1 * (unsigned)n2;
-    // Far from the surface every neighbour distance is phimax: the update is then the same
-    // for every such cell, eikonal(phimax, phimax, phimax, h) (its costliest branch, two
-    // square roots and a division), formed once here by the same code.
-    const float far = jmin(eikonal(phimax, phimax, phimax, h), phimax);
-    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        // 32-bit index arithmetic: a 64-bit division costs more than the cell's update
-        const unsigned row = t / rq;
-        const int q = (int)(t - row * rq);
-        const unsigned kq = row / (unsigned)n2;
-        const int j = (int)(row - kq * (unsigned)n2), k = (int)kq;
-        const int i0 = q * W;
-        const unsigned base = row * (unsigned)n1 + (unsigned)i0;
-        // the wall test (issolidcell, src/flip.jl:64-66) of cells i0-1 .. i0+W and of the
-        // rows at -+y, -+z
-        float pxx[W + 2];
-#pragma unroll
-        for (int m = 0; m < W + 2; m++) {
-            const float px = g.lo[0] + ((float)(i0 - 1 + m) + 0.5f) * dx;
-            pxx[m] = px * px;
-        }
-        const float py = g.lo[1] + ((float)j + 0.5f) * dx, pyp = g.lo[1] + ((float)(j + 1) + 0.5f) * dx,
-                    pym = g.lo[1] + ((float)(j - 1) + 0.5f) * dx;
-        const float pyy = py * py, pyyp = pyp * pyp, pyym = pym * pym;
-        const float pz = g.lo[2] + ((float)k + 0.5f) * dx, pzp = g.lo[2] + ((float)(k + 1) + 0.5f) * dx,
-                    pzm = g.lo[2] + ((float)(k - 1) + 0.5f) * dx;
-        const bool zs = pz < g.floor_z, zsp = pzp < g.floor_z, zsm = pzm < g.floor_z;
-        // the values: the row's cells, -+x beyond them, the rows at -+y, -+z (read only
-        // where the neighbour is in range)
-        float c[W], yp[W], ym[W], zp[W], zm[W];
-        const bool hy = j + 1 < n2, ly = j > 0, hz = k + 1 < n3, lz = k > 0;
-        if constexpr (W == 4) {
-            const float4 a = *reinterpret_cast<const float4*>(phi + base);
-            c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
-            const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 b1 = hy ? *reinterpret_cast<const float4*>(phi + base + sy) : z4;
-            const float4 b2 = ly ? *reinterpret_cast<const float4*>(phi + base - sy) : z4;
-            const float4 b3 = hz ? *reinterpret_cast<const float4*>(phi + base + sz) : z4;
-            const float4 b4 = lz ? *reinterpret_cast<const float4*>(phi + base - sz) : z4;
-            yp[0] = b1.x; yp[1] = b1.y; yp[2] = b1.z; yp[3] = b1.w;
-            ym[0] = b2.x; ym[1] = b2.y; ym[2] = b2.z; ym[3] = b2.w;
-            zp[0] = b3.x; zp[1] = b3.y; zp[2] = b3.z; zp[3] = b3.w;
-            zm[0] = b4.x; zm[1] = b4.y; zm[2] = b4.z; zm[3] = b4.w;
-        } else {
-            c[0] = phi[base];
-            yp[0] = hy ? phi[base + sy] : 0.f;
-            ym[0] = ly ? phi[base - sy] : 0.f;
-            zp[0] = hz ? phi[base + sz] : 0.f;
-            zm[0] = lz ? phi[base - sz] : 0.f;
-        }
-        const float xl = i0 > 0 ? phi[base - 1] : 0.f;
-        const float xr = i0 + W < n1 ? phi[base + W] : 0.f;
-        float o[W];
-        uint8_t ty[W];
-#pragma unroll
-        for (int m = 0; m < W; m++) {
-            const int i = i0 + m;
-            const float cm = c[m];
-            // neighbours in `neighbour`'s order (src/flip.jl:84-92): +x, -x, +y, -y, +z, -z
-            float f[6];
-            bool ok[6];
-            f[0] = m + 1 < W ? c[m + 1 < W ? m + 1 : 0] : xr;
-            f[1] = m > 0 ? c[m > 0 ? m - 1 : 0] : xl;
-            f[2] = yp[m];
-            f[3] = ym[m];
-            f[4] = zp[m];
-            f[5] = zm[m];
-            ok[0] = i + 1 < n1 && !(pxx[m + 2] + pyy > R2 || zs);
-            ok[1] = i > 0 && !(pxx[m] + pyy > R2 || zs);
-            ok[2] = hy && !(pxx[m + 1] + pyyp > R2 || zs);
-            ok[3] = ly && !(pxx[m + 1] + pyym > R2 || zs);
-            ok[4] = hz && !(pxx[m + 1] + pyy > R2 || zsp);
-            ok[5] = lz && !(pxx[m + 1] + pyy > R2 || zsm);
-            const bool solid = pxx[m + 1] + pyy > R2 || zs;
-            float v;
-            if (solid) {
-                // a wall cell takes the lowest value of the water next to it
-                float lowest = cm;
-                bool found = false;
-#pragma unroll
-                for (int e = 0; e < 6; e++)
-                    if (ok[e]) {
-                        lowest = found ? jmin(lowest, f[e]) : f[e];
-                        found = true;
-                    }
-                v = found ? lowest : (cm > phimax ? phimax : (cm < -phimax ? -phimax : cm));
-            } else {
-                const bool inside = cm < 0.0f;
-                bool frozen = false;
-                float ax = phimax, ay = phimax, az = phimax;
-#pragma unroll
-                for (int e = 0; e < 6; e++)
-                    if (ok[e]) {
-                        if ((f[e] < 0.0f) != inside) frozen = true;
-                        const float d = fabsf(f[e]);
-                        if (e < 2) ax = jmin(ax, d);
-                        else if (e < 4) ay = jmin(ay, d);
-                        else az = jmin(az, d);
-                    }
-                if (frozen) {
-                    v = cm;
-                } else {
-                    const float d = (ax == phimax && ay == phimax && az == phimax) ? far
-                                                                                  : jmin(eikonal(ax, ay, az, h), phimax);
-                    v = inside ? -d : d;
-                }
-            }
-            o[m] = v;
-            ty[m] = solid ? SOLID : (v < 0.0f ? LIQUID : AIR);
-        }
-        if constexpr (W == 4) {
-            *reinterpret_cast<float4*>(out + base) = make_float4(o[0], o[1], o[2], o[3]);
-            if (types) *reinterpret_cast<uchar4*>(types + base) = make_uchar4(ty[0], ty[1], ty[2], ty[3]);
-        } else {
-            out[base] = o[0];
-            if (types) types[base] = ty[0];
-        }
+    const int kf = wl.rows[g.n[1]].x;
+    const float far = jmin(eikonal(phimax, phimax, phimax, g.dx), phimax);
+    FOR_CELLS(g.n[0], g.n[1], g.n[2], i, j, k, idx) {
+        bool solid;
+        const float v = reinit_any(g, wl, phi, i, j, k, kf, phimax, far, solid);
+        out[idx] = v;
+        if (types) types[idx] = solid ? SOLID : (v < 0.0f ? LIQUID : AIR);
     }
 }
 
@@ -246,10 +370,8 @@ __global__ void __launch_bounds__(TPB) k_trap_pack(TrapMasks T, const uint8_t* _
             const uint4 v0 = reinterpret_cast<const uint4*>(p)[0], v1 = reinterpret_cast<const uint4*>(p)[1];
             const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
-            for (int q = 0; q < 8; q++)
-#pragma unroll
-                for (int b = 0; b < 4; b++)
-                    if (((w[q] >> (8 * b)) & 0xffu) == AIR) a |= 1u << (4 * q + b);
+            for (int q = 0; q < 8; q++)  // four classes at a time: a byte of ones each, one bit of it kept, added up
+                a |= (((__vcmpeq4(w[q], 0x01010101u * AIR) & 0x08040201u) * 0x01010101u) >> 24) << (4 * q);
         } else {
             const int cnt = T.n1 - i0 < 32 ? T.n1 - i0 : 32;
             for (int b = 0; b < cnt; b++)
