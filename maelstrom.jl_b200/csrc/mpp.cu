@@ -515,6 +515,14 @@ struct Run {
             cudaStreamWaitEvent(c->aux, c->ev_fork, 0);
             s = c->aux;
         }
+        // The fine x and the CG direction start at zero too: the passes add neighbours without looking at
+        // their class, and where an earlier projection of this context had water and this one has
+        // none, nothing else clears them.
+        {
+            const size_t N0 = (size_t)c->grid.n[0] * c->grid.n[1] * c->grid.n[2];
+            cudaMemsetAsync(c->lv[0].x, 0, ms * N0, s);
+            cudaMemsetAsync(c->d, 0, vsize(c->prec) * N0, s);
+        }
         for (int l = 1; l < c->L; l++) {
             const LevelBuf& f = c->lv[l - 1];
             const uint8_t* tf = l == 1 ? in.types : f.types;
