@@ -127,6 +127,7 @@ struct mpp_ctx {
     size_t tflag_bytes;
     Scalars* sc;
     Scalars* sc_host;  // pinned
+    int* turn;         // pinned: the host-driven loop's turn (loop_turn)
     double* partials;
     unsigned* counters;
     std::vector<void*> allocs;
@@ -616,8 +617,11 @@ struct Run {
         end();
     }
     // vcycle! (src/flip.jl:992-1014): z = M^-1 r from zero. with_start = false: the fine
-    // level's start already ran (the CG loop's: after the set-up, and in the step).
-    void vcycle(bool with_start = true) {
+    // level's start already ran (the CG loop's: after the set-up, and in the step). part: HEAD is
+    // the fine level's first colour passes alone, REST what follows them.
+    enum Part { WHOLE, HEAD, REST };
+    static constexpr int HEAD_PASSES = 3;
+    void vcycle(bool with_start = true, Part part = WHOLE) {
         // sweeps of the fine level and of the coarser ones (the reference's one `sweeps`
         // unless sweeps_coarse is set)
         const int swf = c->opts.sweeps, sw = c->opts.sweeps_coarse > 0 ? c->opts.sweeps_coarse : swf;
@@ -628,13 +632,20 @@ struct Run {
         for (int q = 0; q < swf; q++) { down0.push_back(0); down0.push_back(1); }
         down0.erase(down0.begin());
         for (int q = 0; q < swf; q++) { up0.push_back(1); up0.push_back(0); }
+        const int nhead = std::min<int>(HEAD_PASSES, (int)down0.size());
+        if (part == HEAD) {
+            down0.resize(nhead);
+            smooth(0, down0, true);
+            return;
+        }
+        if (part == REST) down0.erase(down0.begin(), down0.begin() + nhead);
         const int lb = c->lb;
         const int ls = c->cmg_ls > 0 ? c->cmg_ls : lb;  // levels ls .. L-1 in the cluster
         for (int l = 0; l < ls; l++) {
             if (l == 0 && with_start) start0();  // the coarser levels' starts ride on the restriction
             // b of the level's first pass waits for the preceding kernel where that kernel wrote
             // it: the restriction that started a coarse level, the step that started level 0
-            smooth(l, l == 0 ? down0 : down, l > 0 || !with_start);
+            smooth(l, l == 0 ? down0 : down, l > 0 || (!with_start && part == WHOLE));
             beg(F_RESID, l);
             if (vec(l)) launch(k_residual_v8<Pr>, grid_res((const void*)k_residual_v8<Pr>, l), TPB, 0, s, view<M>(c, l));
             else launch(k_residual<Pr>, grid_tiles(c, l), TPB, 0, s, view<M>(c, l));
@@ -679,8 +690,9 @@ struct Run {
     // The next V-cycle's fine start is part of the step: the vector step writes it (the b
     // it has just formed, over the stored reciprocal diagonal or diagonal), otherwise the start
     // kernel follows the step; the set-up is followed by one (record_prologue).
-    void body(V* P, cudaGraphConditionalHandle cond, int use_cond) {
-        vcycle(false);
+    void body(V* P, cudaGraphConditionalHandle cond, int use_cond, Part part = WHOLE) {
+        vcycle(false, part);
+        if (part == HEAD) return;
         const bool v = vec(0);
         beg(F_DOT, 0);
         if (v)
@@ -949,6 +961,7 @@ int write_params(mpp_ctx* c, float volume0, double dt, double recover, int proje
     p.maxiter = c->opts.fallback ? std::min(c->opts.maxiter, c->opts.cg_maxiter_with_fallback) : c->opts.maxiter;
     p.project = project;
     p.gamma = gamma;
+    p.turn = c->opts.graph || c->prof_on ? nullptr : c->turn;
     CK(cudaMemcpyAsync(&c->sc->p, &c->sc_host->p, sizeof(Params), cudaMemcpyHostToDevice, s));
     return MPP_OK;
 }
@@ -957,6 +970,29 @@ int read_state(mpp_ctx* c, cudaStream_t s) {
     CK(cudaMemcpyAsync(&c->sc_host->s, &c->sc->s, sizeof(State), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     return MPP_OK;
+}
+
+// The host-driven loop's turn after step `it` (0: the set-up), as loop_turn tells it.
+int wait_turn(mpp_ctx* c, cudaStream_t s, int it, bool& go) {
+    const volatile int* turn = c->turn;
+    for (unsigned spins = 1;; spins++) {
+        const int t = *turn;
+        if (t >= 0 && ((t & 1) || (t >> 1) >= it)) {
+            go = !(t & 1);
+            return MPP_OK;
+        }
+        if (spins % 4096 == 0) {  // the stream ended without a turn: an error, or the word is on its way
+            const cudaError_t q = cudaStreamQuery(s);
+            if (q != cudaSuccess && q != cudaErrorNotReady) {
+                set_err("the solve's stream: %s", cudaGetErrorString(q));
+                return MPP_ERR_CUDA;
+            }
+            if (q == cudaSuccess && (*turn < 0 || (!(*turn & 1) && (*turn >> 1) < it))) {
+                set_err("the solve's kernels ended without the loop's turn");
+                return MPP_ERR_CUDA;
+            }
+        }
+    }
 }
 
 struct Call {
@@ -1320,12 +1356,26 @@ int solve(mpp_ctx* c, const Call& k, cudaStream_t s) {
         launched = ge->g_prologue + (int64_t)ge->g_body * c->sc_host->s.it + ge->g_epilogue;
     } else {
         Run<Pr> run{c, s};
-        record_prologue<Pr>(run, k, 0, 0);
-        if (int e = read_state(c, s)) return e;
         V* P = std::is_same<V, double>::value ? (V*)c->Pd : (V*)k.P;
-        while (!c->sc_host->s.done) {
-            run.body(P, 0, 0);
+        if (c->prof_on) {
+            record_prologue<Pr>(run, k, 0, 0);
             if (int e = read_state(c, s)) return e;
+            while (!c->sc_host->s.done) {
+                run.body(P, 0, 0);
+                if (int e = read_state(c, s)) return e;
+            }
+        } else {
+            // the next V-cycle's first passes go out before the loop's turn is known: after the last
+            // step they only write the V-cycle's own x
+            *c->turn = -1;
+            record_prologue<Pr>(run, k, 0, 0);
+            for (int it = 0;; it++) {
+                run.body(P, 0, 0, Run<Pr>::HEAD);
+                bool go = false;
+                if (int e = wait_turn(c, s, it, go)) return e;
+                if (!go) break;
+                run.body(P, 0, 0, Run<Pr>::REST);
+            }
         }
         record_epilogue<Pr>(run, k);
         if (int e = read_state(c, s)) return e;
@@ -1718,6 +1768,7 @@ int mpp_ctx_destroy(mpp_ctx* c) {
     if (c->trap_graph) cudaGraphDestroy(c->trap_graph);
     for (void* p : c->allocs) cudaFree(p);
     if (c->sc_host) cudaFreeHost(c->sc_host);
+    if (c->turn) cudaFreeHost(c->turn);
     if (c->fgd_host) cudaFreeHost(c->fgd_host);
     if (c->cap) cudaStreamDestroy(c->cap);
     if (c->aux) cudaStreamDestroy(c->aux);
@@ -1788,6 +1839,7 @@ int mpp_ctx_create(mpp_ctx** out, const mpp_grid* g, const mpp_opts* o) {
     c->bytes = 0;
     c->launches = 0;
     c->sc_host = nullptr;
+    c->turn = nullptr;
     c->cap = nullptr;
     c->aux = nullptr;
     c->ev_fork = c->ev_join = nullptr;
@@ -1959,6 +2011,7 @@ int mpp_ctx_create(mpp_ctx** out, const mpp_grid* g, const mpp_opts* o) {
     if ((e = alloc(c, (void**)&c->partials, sizeof(double) * MAXK * (size_t)c->nsm * MAXBLOCKS_PER_SM))) return fail(e);
     if ((e = alloc(c, (void**)&c->counters, sizeof(unsigned) * NCOUNTERS))) return fail(e);
     ce = cudaMallocHost((void**)&c->sc_host, sizeof(Scalars));
+    if (ce == cudaSuccess) ce = cudaMallocHost((void**)&c->turn, sizeof(int));
     if (ce != cudaSuccess) {
         set_err("cudaMallocHost: %s", cudaGetErrorString(ce));
         return fail(MPP_ERR_NOMEM);

@@ -408,7 +408,10 @@ __global__ void __launch_bounds__(SPT) k_sp_update(Topo t, const uint8_t* tf, co
     pdl_wait();
     pdl_trigger();
     if (st->done) {
-        if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (use_cond) cudaGraphSetConditional(cond, 0u);
+            else sp_turn(st);
+        }
         return;
     }
     const float alpha = st->alpha, ma = -alpha;
@@ -438,6 +441,7 @@ __global__ void __launch_bounds__(SPT) k_sp_update(Topo t, const uint8_t* tf, co
             st->done = 1;
         }
         if (use_cond) cudaGraphSetConditional(cond, st->done ? 0u : 1u);
+        else sp_turn(st);
     }
 }
 
@@ -733,6 +737,7 @@ struct mpp_sparse_ctx {
     bool fg_alloc;
     SpState* st;
     SpState* st_host;
+    int* turn;          // pinned: the host-driven loop's turn (sp_turn)
     double* dres;       // dot results (FGMRES)
     double* dres_host;
     double* partials;
@@ -957,12 +962,16 @@ struct SpRun {
         }
     }
     // vcycle! (src/sflip.jl:1722-1764): z = M^-1 r
+    // part: HEAD is the first sweep pair alone, REST what follows it.
+    enum Part { WHOLE, HEAD, REST };
     void vcycle(const uint8_t* tf, float* zf, float* zc, const float* rf, const float* rc, int sweeps, int coarse,
-                float boost) {
+                float boost, Part part = WHOLE) {
         const Topo& t = c->t;
         const Comp L0 = comp0(c, tf), L1 = comp1(c);
         const Split s0 = split_for(c, (int64_t)t.nslots * BCELLS), s1 = split_for(c, (int64_t)t.nslots * BCELLS1);
-        smooth<16>(L0, zf, zc, rf, rc, c->tmf, c->tmc, sweeps, true);
+        if (part != REST) smooth<16>(L0, zf, zc, rf, rc, c->tmf, c->tmc, part == HEAD ? 1 : sweeps, true);
+        else if (sweeps > 1) smooth<16>(L0, zf, zc, rf, rc, c->tmf, c->tmc, sweeps - 1, false);
+        if (part == HEAD) return;
         const Split sb = split_blk(c);
         sp_launch(k_sp_blk<BOP_RES, SrcX>, dim3(sb.g), SPT, s, t, L0, (const uint16_t*)c->code0,
                   (const float*)c->dg0, c->res0f, c->res0c, SrcX{zf, zc}, rf, rc,
@@ -1038,10 +1047,12 @@ struct SpRun {
         nk += 2;
     }
     // the rotated loop body: the V-cycle of the new residual, beta, d, then q, alpha, the update
-    void cg_body(const mpp_sparse_basin* b, const mpp_sparse_opts* o, cudaGraphConditionalHandle cond, int use_cond) {
+    void cg_body(const mpp_sparse_basin* b, const mpp_sparse_opts* o, cudaGraphConditionalHandle cond, int use_cond,
+                 Part part = WHOLE) {
         const Topo& t = c->t;
         const Split sv = split_vec(c);
-        vcycle(b->types_f, c->zf, c->zc, c->rf, c->rc, o->sweeps, o->coarse, o->boost);
+        vcycle(b->types_f, c->zf, c->zc, c->rf, c->rc, o->sweeps, o->coarse, o->boost, part);
+        if (part == HEAD) return;
         sp_launch(k_sp_dot2, dim3(sv.g), SPT, s, t, b->types_f, (const uint8_t*)c->cmask, (const float*)c->zf, (const float*)c->zc,
                   (const float*)c->rf, (const float*)c->rc, (const float*)c->rof, (const float*)c->roc, c->st,
                   c->partials, c->counters + SCNT_DOT2, (const uint32_t*)c->pm, sv.gf);
@@ -1068,6 +1079,29 @@ int read_state(mpp_sparse_ctx* c, cudaStream_t s) {
     SCK(cudaMemcpyAsync(c->st_host, c->st, sizeof(SpState), cudaMemcpyDeviceToHost, s));
     SCK(cudaStreamSynchronize(s));
     return MPP_OK;
+}
+
+// The host-driven loop's turn after step `it`, as sp_turn tells it.
+int wait_turn(mpp_sparse_ctx* c, cudaStream_t s, int it, bool& go) {
+    const volatile int* turn = c->turn;
+    for (unsigned spins = 1;; spins++) {
+        const int t = *turn;
+        if (t >= 0 && ((t & 1) || (t >> 1) >= it)) {
+            go = !(t & 1);
+            return MPP_OK;
+        }
+        if (spins % 4096 == 0) {  // the stream ended without a turn: an error, or the word is on its way
+            const cudaError_t q = cudaStreamQuery(s);
+            if (q != cudaSuccess && q != cudaErrorNotReady) {
+                sp_err("the solve's stream: %s", cudaGetErrorString(q));
+                return MPP_ERR_CUDA;
+            }
+            if (q == cudaSuccess && (*turn < 0 || (!(*turn & 1) && (*turn >> 1) < it))) {
+                sp_err("the solve's kernels ended without the loop's turn");
+                return MPP_ERR_CUDA;
+            }
+        }
+    }
 }
 
 // a dot product over the unknowns, read back (FGMRES)
@@ -1270,23 +1304,31 @@ int solve(mpp_sparse_ctx* c, SpRun& run, const mpp_sparse_basin* b, const mpp_sp
     SpState init = {};
     init.tol = o->tol;
     init.maxiter = fb ? std::min(o->cg_maxiter, o->maxiter) : o->maxiter;
+    init.turn = o->graph ? nullptr : c->turn;
     // keep project!'s volume terms already on the device: write only the loop's fields
-    SCK(cudaMemcpyAsync(&c->st->tol, &init.tol, sizeof(float) * 2, cudaMemcpyHostToDevice, run.s));
+    SCK(cudaMemcpyAsync(&c->st->tol, &init.tol, offsetof(SpState, bnorm), cudaMemcpyHostToDevice, run.s));
+    *c->turn = -1;
     run.cg_prologue(b, o, 0, 0);
-    if (int e = read_state(c, run.s)) return e;
-    if (!c->st_host->done) {
-        if (o->graph) {
+    if (!o->graph) {
+        // the next V-cycle's first sweep goes out before the loop's turn is known: after the last
+        // step it only writes the V-cycle's own z
+        for (int it = 1;; it++) {
+            run.cg_body(b, o, 0, 0, SpRun::HEAD);
+            bool go = false;
+            if (int e = wait_turn(c, run.s, it, go)) return e;
+            if (!go) break;
+            run.cg_body(b, o, 0, 0, SpRun::REST);
+        }
+        if (int e = read_state(c, run.s)) return e;
+    } else {
+        if (int e = read_state(c, run.s)) return e;
+        if (!c->st_host->done) {
             cudaGraphExec_t ge;
             int64_t bk;
             if (int e = loop_graph(c, b, o, &ge, &bk)) return e;
             SCK(cudaGraphLaunch(ge, run.s));
             if (int e = read_state(c, run.s)) return e;
             run.nk += bk * (c->st_host->it - 1);
-        } else {
-            while (!c->st_host->done) {
-                run.cg_body(b, o, 0, 0);
-                if (int e = read_state(c, run.s)) return e;
-            }
         }
     }
     SCK(cudaGetLastError());
@@ -1448,6 +1490,7 @@ int mpp_sparse_ctx_create(mpp_sparse_ctx** out, const mpp_sparse_grid* g, int32_
     if (int e2 = sp_alloc_n(c, &c->partials, (std::max((int64_t)capacity, cap8) + cap8) * 2)) return fail(e2);
     if (int e2 = sp_alloc_n(c, &c->counters, SCNT_N)) return fail(e2);
     if (cudaMallocHost((void**)&c->st_host, sizeof(SpState)) != cudaSuccess ||
+        cudaMallocHost((void**)&c->turn, sizeof(int)) != cudaSuccess ||
         cudaMallocHost((void**)&c->dres_host, sizeof(double)) != cudaSuccess) {
         sp_err("cudaMallocHost failed");
         return fail(MPP_ERR_NOMEM);
@@ -1465,6 +1508,7 @@ int mpp_sparse_ctx_destroy(mpp_sparse_ctx* c) {
     drop_graph(c);
     for (void* p : c->allocs) cudaFree(p);
     if (c->st_host) cudaFreeHost(c->st_host);
+    if (c->turn) cudaFreeHost(c->turn);
     if (c->dres_host) cudaFreeHost(c->dres_host);
     if (c->cap) cudaStreamDestroy(c->cap);
     delete c;

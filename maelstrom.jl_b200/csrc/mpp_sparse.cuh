@@ -990,6 +990,7 @@ __global__ void __launch_bounds__(SPT) k_sp_prolong21(Topo t, float* xf, float* 
 struct SpState {
     float tol;
     int maxiter;
+    int* turn;  // pinned host memory for a loop driven by the host (null: the graph's loop): see sp_turn
     float bnorm, target, rnorm, rho, alpha, beta, den;
     int status, it, done;
     float vol, gamma;  // project!'s volume and volume-control divergence
@@ -997,6 +998,14 @@ struct SpState {
     int pad;
     double dt, recover;
 };
+
+// Whether the CG goes on after a step, told to the host that drives the loop: 2 * iteration + stop
+// (the host has the next V-cycle's first sweep under way meanwhile).
+__device__ __forceinline__ void sp_turn(const SpState* st) {
+    if (!st->turn) return;
+    __threadfence_system();
+    *reinterpret_cast<volatile int*>(st->turn) = 2 * st->it + (st->done ? 1 : 0);
+}
 
 // The inner (src/sflip.jl:1794-1805) masks: LIQUID fine cells of slots in use; LIQUID coarse
 // cells outside fine blocks.

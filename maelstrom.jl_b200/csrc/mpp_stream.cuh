@@ -121,7 +121,7 @@ __device__ __forceinline__ void advance_finish(Scalars* sc, const double (&acc)[
         S.status = ST_NOT_CONVERGED;
         S.done = 1;
     }
-    set_cond(cond, use_cond, !S.done);
+    loop_turn(sc, cond, use_cond, !S.done);
 }
 
 // ---- the V-cycle (src/flip.jl:992-1014) on row-split levels ----
@@ -772,7 +772,7 @@ __device__ __forceinline__ void advance_v8_dev(Lev<typename Pr::M> L, typename P
     pdl_wait();
     pdl_trigger();
     if (sc->s.done) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(cond, use_cond, 0);
+        if (blockIdx.x == 0 && threadIdx.x == 0) loop_turn(sc, cond, use_cond, 0);
         return;
     }
     const C beta = (C)sc->s.beta, alpha = (C)sc->s.alpha;
@@ -1192,7 +1192,7 @@ __device__ __forceinline__ void advance_dev(Lev<typename Pr::M> L, typename Pr::
     pdl_trigger();
     using C = typename Pr::C;
     if (sc->s.done) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(cond, use_cond, 0);
+        if (blockIdx.x == 0 && threadIdx.x == 0) loop_turn(sc, cond, use_cond, 0);
         return;
     }
     const C beta = (C)sc->s.beta, alpha = (C)sc->s.alpha;
@@ -1251,7 +1251,7 @@ __device__ __forceinline__ void advance_dev(Lev<typename Pr::M> L, typename Pr::
             S.status = ST_NOT_CONVERGED;
             S.done = 1;
         }
-        set_cond(cond, use_cond, !S.done);
+        loop_turn(sc, cond, use_cond, !S.done);
     }
 }
 template <class Pr>
