@@ -249,6 +249,7 @@ ClArgs<M> cluster_args(const mpp_ctx* c, int sweeps) {
     a.orb = c->cmg_orb;
     a.ogi = c->cmg_ogi;
     a.fault = &c->sc->s.fault;
+    a.tries = 1 << 16;
     a.cl = c->bot.lv[c->bot.nl - 1];
     for (int q = 0; q <= a.nl; q++) a.s[q] = c->cmg_lev[q];
     for (int q = 0; q < a.nl; q++) a.g[q] = view<M>(c, c->cmg_ls + q);
