@@ -151,7 +151,7 @@ struct mpp_ctx {
     size_t bot_smem, restrict_smem;
     void* botb;  // level lb's right-hand side (natural order, stencil precision)
     // levels cmg_ls .. L-1 resident in one cluster of cmg_cs CTAs (k_cluster), when cmg_ls > 0
-    int cmg_ls, cmg_cs;
+    int cmg_ls, cmg_cs, cmg_tries;
     size_t cmg_smem;
     ClLev cmg_lev[CL_MAXLEV + 1];
     int cmg_nd, cmg_nact;  // levels spread over the cluster, CTAs that hold planes of them
@@ -249,7 +249,7 @@ ClArgs<M> cluster_args(const mpp_ctx* c, int sweeps) {
     a.orb = c->cmg_orb;
     a.ogi = c->cmg_ogi;
     a.fault = &c->sc->s.fault;
-    a.tries = 1 << 16;
+    a.tries = c->cmg_tries;
     a.cl = c->bot.lv[c->bot.nl - 1];
     for (int q = 0; q <= a.nl; q++) a.s[q] = c->cmg_lev[q];
     for (int q = 0; q < a.nl; q++) a.g[q] = view<M>(c, c->cmg_ls + q);
@@ -973,6 +973,16 @@ int read_state(mpp_ctx* c, cudaStream_t s) {
     return MPP_OK;
 }
 
+// The error of a bounded device wait that gave up (the state read back).
+int check_fault(const mpp_ctx* c, int basin = -1) {
+    const int f = c->sc_host->s.fault;
+    if (f == 0) return MPP_OK;
+    const char* what = f == FAULT_CLUSTER ? "halo exchange of the small levels' cluster" : "TMA pipeline";
+    if (basin >= 0) set_err("basin %d: a bounded device wait (%s) gave up; results are not valid", basin, what);
+    else set_err("a bounded device wait (%s) gave up; results are not valid", what);
+    return MPP_ERR_CUDA;
+}
+
 // The host-driven loop's turn after step `it` (0: the set-up), as loop_turn tells it.
 int wait_turn(mpp_ctx* c, cudaStream_t s, int it, bool& go) {
     const volatile int* turn = c->turn;
@@ -1214,7 +1224,7 @@ int fgmres(mpp_ctx* c, cudaStream_t s, typename Pr::V* P, int& its, int& status)
 // true residual meets tol; else zero P if that residual is nonfinite or above 2|b|, run FGMRES,
 // and then (project!) the gradient update.
 template <class Pr>
-int fallback_and_finish(mpp_ctx* c, const Call& k, cudaStream_t s) {
+int fallback_and_finish(mpp_ctx* c, const Call& k, cudaStream_t s, int basin = -1) {
     using V = typename Pr::V;
     State& S = c->sc_host->s;
     c->fg_used = 0;
@@ -1231,6 +1241,8 @@ int fallback_and_finish(mpp_ctx* c, const Call& k, cudaStream_t s) {
         }
         int its = 0, st = 0;
         if (int e = fgmres<Pr>(c, s, P, its, st)) return e;
+        if (int e = read_state(c, s)) return e;  // its V-cycles' waits
+        if (int e = check_fault(c, basin)) return e;
         c->fg_used = 1;
         c->fg_its = its;
         S.status = st;
@@ -1385,10 +1397,7 @@ int solve(mpp_ctx* c, const Call& k, cudaStream_t s) {
     }
     CK(cudaGetLastError());
     c->launches += launched;
-    if (c->sc_host->s.fault) {
-        set_err("a bounded device wait (TMA pipeline) gave up; results are not valid");
-        return MPP_ERR_CUDA;
-    }
+    if (int e = check_fault(c)) return e;
     c->fg_used = c->fg_its = 0;
     if (c->opts.fallback) return fallback_and_finish<Pr>(c, k, s);
     return MPP_OK;
@@ -1571,12 +1580,15 @@ int build_walls(mpp_ctx* c) {
 
 // The levels of k_cluster: from the first one of at most CL_CELLS cells whose planes (and those of
 // every smaller level) fit the shared memory of a cluster's CTAs, down to the coarsest. In the
-// environment MPP_CMG=0 keeps the per-level launches and MPP_CMG_MAXCELLS sets the size bound.
+// environment MPP_CMG=0 keeps the per-level launches, MPP_CMG_MAXCELLS sets the size bound and
+// MPP_CMG_TRIES the polls after which an exchange wait gives up (0: all of them, at once).
 int build_cmg(mpp_ctx* c) {
     c->cmg_ls = 0;
     c->cmg_cs = 0;
     c->cmg_nd = c->cmg_nact = 0;
     c->cmg_smem = 0;
+    c->cmg_tries = 1 << 16;
+    if (const char* ct = getenv("MPP_CMG_TRIES")) c->cmg_tries = std::max(0, atoi(ct));
     const char* env = getenv("MPP_CMG");
     if ((env && !strcmp(env, "0")) || c->lb < 2) return MPP_OK;
     int64_t maxcells = CL_CELLS;
@@ -2422,15 +2434,12 @@ int mpp_batch_project(mpp_batch* b, const mpp_basin_arrays* basins, double dt, d
         mpp_ctx* c = b->ctx[i];
         const int* k3 = &b->counts[3 * i];
         c->launches += k3[0] + (int64_t)k3[1] * c->sc_host->s.it + k3[2];
-        if (c->sc_host->s.fault) {
-            set_err("basin %d: a bounded device wait (TMA pipeline) gave up; results are not valid", i);
-            return MPP_ERR_CUDA;
-        }
+        if (int e = check_fault(c, i)) return e;
         c->fg_used = c->fg_its = 0;
         if (c->opts.fallback) {
             const mpp_basin_arrays& a = basins[i];
             Call k{1, a.u, a.v, a.w, a.fu, a.fv, a.fw, a.P, nullptr, a.types, a.phi};
-            int e = dispatch(c->prec, [&](auto pr) { return fallback_and_finish<decltype(pr)>(c, k, s); });
+            int e = dispatch(c->prec, [&](auto pr) { return fallback_and_finish<decltype(pr)>(c, k, s, i); });
             if (e) return e;
         }
         if (results) fill_result(c, &results[i], c->launches - launches0[i]);
@@ -3008,13 +3017,14 @@ int mpp_vcycle(mpp_ctx* c, float* z, const float* r, const uint8_t* types, const
         const int64_t N = (int64_t)c->grid.n[0] * c->grid.n[1] * c->grid.n[2];
         const size_t ms = msize(c->prec);
         CK(cudaMemsetAsync(c->lv[0].x, 0, ms * N, s));
+        CK(cudaMemsetAsync(&c->sc->s.fault, 0, sizeof(int), s));
         launch(k_to_split<M, float>, grid_cells(c, N), TPB, 0, s, fine_layout(c), (M*)c->lv[0].b, r);
         run.vcycle();
         launch(k_from_split<float, M>, grid_cells(c, N), TPB, 0, s, fine_layout(c), z, (const M*)c->lv[0].x);
         CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(s));
+        if (int e = read_state(c, s)) return e;
         c->launches += run.nk + 2;
-        return MPP_OK;
+        return check_fault(c);
     });
 }
 

@@ -32,7 +32,7 @@ struct State {
     int status;      // MPP_* status
     int it;          // CG iterations done
     int done;        // 1 once the loop must stop
-    int fault;       // a bounded device wait gave up (the host reports an error)
+    int fault;       // a bounded device wait gave up, FAULT_* says which (the host reports an error)
     int pad;
 };
 
@@ -41,6 +41,7 @@ struct Scalars {
     State s;
 };
 
+enum { FAULT_TMA = 1, FAULT_CLUSTER = 2 };
 enum { ST_OK = 0, ST_NOT_CONVERGED = 1, ST_NONFINITE = 2, ST_INDEFINITE = 3, ST_BREAKDOWN = 4 };
 
 __device__ __forceinline__ bool finite_d(double x) { return isfinite(x); }

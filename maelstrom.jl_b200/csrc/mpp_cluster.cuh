@@ -390,7 +390,7 @@ struct ClRun {
         if (!done) {
             off = true;
             *(volatile int*)&sh.dead = 1;
-            *a.fault = 1;
+            *a.fault = FAULT_CLUSTER;
         }
     }
 

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(TPB) k_rbgs_tma(Lev<typename Pr::M> L, int col
     }
     if (bad) {
         if (threadIdx.x == 0) {
-            atomicExch(fault, 1);
+            atomicExch(fault, FAULT_TMA);
             // copies still in flight: tiles i .. i + S - 1 that were issued
             for (int q = i; q < issued; q++) mbar_wait_bounded(&full[q % S], (uint32_t)((q / S) & 1));
         }
