@@ -860,6 +860,10 @@ struct SpRun {
     // whether the V-cycle takes every piece: its input may be nonzero off the water (the V-cycle
     // entry's is the caller's), or its output array is not one that the operator clears there
     bool all_pieces = false;
+    // whether the right-hand side may be nonzero off the water (the pressure entry's is the caller's): the
+    // V-cycle's residual, which hands it to the restriction from every cell that is not SOLID, then takes
+    // every piece; the sweeps leave zeros there, and every other pass's sums are over the water alone
+    bool rhs_any = false;
     const uint32_t* pm() const { return all_pieces ? c->pm_all : c->pm; }
     int ps() const { return all_pieces ? 0 : 32; }
 
@@ -975,7 +979,7 @@ struct SpRun {
         const Split sb = split_blk(c);
         sp_launch(k_sp_blk<BOP_RES, SrcX>, dim3(sb.g), SPT, s, t, L0, (const uint16_t*)c->code0,
                   (const float*)c->dg0, c->res0f, c->res0c, SrcX{zf, zc}, rf, rc,
-                  pm(), ps(), sb.gf);
+                  rhs_any ? c->pm_all : pm(), rhs_any ? 0 : ps(), sb.gf);
         sp_launch(k_sp_restrict01, dim3(grid1((int64_t)t.nslots * BCELLS1)), SPT, s, t, c->b1f,
                   (const float*)c->res0f);
         nk += 2;
@@ -1257,10 +1261,10 @@ int drop_graph(mpp_sparse_ctx* c) {
 }
 
 // The CG loop (after the prologue) as a graph: one conditional WHILE node over the rotated body.
-int loop_graph(mpp_sparse_ctx* c, const mpp_sparse_basin* b, const mpp_sparse_opts* o, cudaGraphExec_t* out,
-               int64_t* body_kernels) {
+int loop_graph(mpp_sparse_ctx* c, const mpp_sparse_basin* b, const mpp_sparse_opts* o, bool rhs_any,
+               cudaGraphExec_t* out, int64_t* body_kernels) {
     const void* key[12] = {b->slot, b->where, b->types_f, b->types_c, b->P_f, b->P_c, b->phi_f, b->phi_c,
-                           (const void*)(intptr_t)b->nslots, nullptr, nullptr, nullptr};
+                           (const void*)(intptr_t)b->nslots, (const void*)(intptr_t)rhs_any, nullptr, nullptr};
     const int opt[4] = {o->sweeps, o->coarse, (int)(o->boost * 1024.0f), 0};
     if (c->gexec && memcmp(key, c->gkey, sizeof(key)) == 0 && memcmp(opt, c->gopt, sizeof(opt)) == 0 &&
         o->boost == (float)opt[2] / 1024.0f) {
@@ -1283,6 +1287,7 @@ int loop_graph(mpp_sparse_ctx* c, const mpp_sparse_basin* b, const mpp_sparse_op
     SCK(cudaGraphAddNode(&cnode, g, nullptr, 0, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     SpRun run{c, c->cap};
+    run.rhs_any = rhs_any;
     SCK(cudaStreamBeginCaptureToGraph(c->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     run.cg_body(b, o, cond, 1);
     const cudaError_t le = cudaGetLastError();
@@ -1325,7 +1330,7 @@ int solve(mpp_sparse_ctx* c, SpRun& run, const mpp_sparse_basin* b, const mpp_sp
         if (!c->st_host->done) {
             cudaGraphExec_t ge;
             int64_t bk;
-            if (int e = loop_graph(c, b, o, &ge, &bk)) return e;
+            if (int e = loop_graph(c, b, o, run.rhs_any, &ge, &bk)) return e;
             SCK(cudaGraphLaunch(ge, run.s));
             if (int e = read_state(c, run.s)) return e;
             run.nk += bk * (c->st_host->it - 1);
@@ -1607,6 +1612,7 @@ int mpp_sparse_pressure(mpp_sparse_ctx* c, const mpp_sparse_basin* b, const floa
     if (int e = check_opts(o)) return e;
     cudaStream_t s = (cudaStream_t)stream;
     SpRun run{c, s};
+    run.rhs_any = true;
     run.operator_(b);
     const int64_t nf = (int64_t)b->nslots * BCELLS;
     SCK(cudaMemcpyAsync(c->bf, bf, sizeof(float) * (size_t)nf, cudaMemcpyDefault, s));
