@@ -14,30 +14,11 @@
 #pragma once
 
 #include "mpp_common.cuh"
+#include "mpp_div.cuh"
 
 namespace mpp {
 
 constexpr int RB_CELLS = 1024, RB_HALF = RB_CELLS / 2;
-
-// a / d, rounded as the IEEE division, for rd = 1 / d rounded: the quotient estimate a rd and
-// its residual, exact in one fused multiply-add, corrected (P. Markstein, IBM J. Res. Dev. 34,
-// 1990: a faithful estimate corrected so is the rounded quotient). There is no test for operands
-// whose residual leaves the normal range, because a branch in the loop costs as much as the
-// division it avoids (157 against 105 cycles a half-sweep at 128 threads; the division itself
-// 144): below 2^-100 a quotient may be one unit of the last place off, and an infinite a gives NaN,
-// which the solves' nonfinite test catches like the infinity.
-// div_small: d = 1 .. 6, a level's count of open faces. One correction rounds every mantissa right
-// (all 2^23 of them checked for each d).
-__device__ __forceinline__ float div_small(float a, float d, float rd) {
-    const float q = a * rd;
-    return fmaf(fmaf(-q, d, a), rd, q);
-}
-// div_rn: any d of ordinary size, in [2^-30, 2^30]; the first correction makes the estimate faithful.
-__device__ __forceinline__ float div_rn(float a, float d, float rd) {
-    float q = a * rd;
-    q = fmaf(fmaf(-q, d, a), rd, q);
-    return fmaf(fmaf(-q, d, a), rd, q);
-}
 
 // Shared memory of the solve: x by colour (RB_HALF places each, then a zero and a spare place), each cell's place
 // and the lists of each colour's cells.

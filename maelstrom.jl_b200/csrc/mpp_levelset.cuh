@@ -28,7 +28,7 @@
 #pragma once
 
 #include "mpp_base.cuh"
-#include "mpp_coarsest.cuh"
+#include "mpp_div.cuh"
 
 namespace mpp {
 
