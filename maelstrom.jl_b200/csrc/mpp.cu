@@ -952,7 +952,9 @@ struct GroupRun {
 };
 static_assert(sizeof(Grp<GCluster<double>>) < 32000, "a group launch's arguments fit the kernel parameter space");
 
-int write_params(mpp_ctx* c, float volume0, double dt, double recover, int project, float gamma, cudaStream_t s) {
+// host_loop: the call may drive its CG loop from the host (a batch's loops are graph nodes)
+int write_params(mpp_ctx* c, float volume0, double dt, double recover, int project, float gamma, cudaStream_t s,
+                 bool host_loop = true) {
     Params& p = c->sc_host->p;
     p.volume0 = volume0;
     p.tol = c->opts.tol;
@@ -962,7 +964,7 @@ int write_params(mpp_ctx* c, float volume0, double dt, double recover, int proje
     p.maxiter = c->opts.fallback ? std::min(c->opts.maxiter, c->opts.cg_maxiter_with_fallback) : c->opts.maxiter;
     p.project = project;
     p.gamma = gamma;
-    p.turn = c->opts.graph || c->prof_on ? nullptr : c->turn;
+    p.turn = host_loop && !c->opts.graph && !c->prof_on ? c->turn : nullptr;
     CK(cudaMemcpyAsync(&c->sc->p, &c->sc_host->p, sizeof(Params), cudaMemcpyHostToDevice, s));
     return MPP_OK;
 }
@@ -2370,7 +2372,7 @@ int mpp_batch_project(mpp_batch* b, const mpp_basin_arrays* basins, double dt, d
         mpp_ctx* c = b->ctx[i];
         launches0[i] = c->launches;
         CK(cudaMemsetAsync(&c->sc->s.fault, 0, sizeof(int), s));
-        if (int e = write_params(c, basins[i].volume0, dt, recover, 1, 0.f, s)) return e;
+        if (int e = write_params(c, basins[i].volume0, dt, recover, 1, 0.f, s, false)) return e;
     }
     if (!b->exec || key != b->key) {
         batch_drop_graph(b);
