@@ -621,7 +621,11 @@ struct Run {
     // level's start already ran (the CG loop's: after the set-up, and in the step). part: HEAD is
     // the fine level's first colour passes alone, REST what follows them.
     enum Part { WHOLE, HEAD, REST };
-    static constexpr int HEAD_PASSES = 3;
+    // How many: enough to last while the loop's turn travels, since the ones after the last step are thrown
+    // away. Up to 128^3 a pass is 2-5 us and three are as good as any number (1, 2, 3, 6 of them: 64^3 717,
+    // 708, 698, 694 us a projection; 96^3 1072, 1058, 1058, 1058; 128^3 1228, 1210, 1211, 1211); from
+    // about 160^3 one pass lasts (192 x 160 x 160 1938, 1942, 1945, 1946; 256^3 4492, 4512, 4523, 4524).
+    int head_passes() const { return (int64_t)c->grid.n[0] * c->grid.n[1] * c->grid.n[2] >= (int64_t)1 << 22 ? 1 : 3; }
     void vcycle(bool with_start = true, Part part = WHOLE) {
         // sweeps of the fine level and of the coarser ones (the reference's one `sweeps`
         // unless sweeps_coarse is set)
@@ -633,7 +637,7 @@ struct Run {
         for (int q = 0; q < swf; q++) { down0.push_back(0); down0.push_back(1); }
         down0.erase(down0.begin());
         for (int q = 0; q < swf; q++) { up0.push_back(1); up0.push_back(0); }
-        const int nhead = std::min<int>(HEAD_PASSES, (int)down0.size());
+        const int nhead = std::min<int>(head_passes(), (int)down0.size());
         if (part == HEAD) {
             down0.resize(nhead);
             smooth(0, down0, true);
