@@ -4,7 +4,8 @@
 
 ``-fmad=false`` keeps every a*b+c as two roundings, so the FP32 kernels round exactly
 as the reference's Float32 code; the kernels are bandwidth-bound, so the lost FMA
-throughput costs nothing measurable.
+throughput costs nothing measurable. ``-ffp-contract=off`` does the same for host code (the
+wall ranges of the level-set passes are host Float32 that has to round as the device's).
 """
 from __future__ import annotations
 
@@ -31,7 +32,7 @@ def nvcc() -> str:
 
 def flags(verbose: bool = False) -> list:
     f = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-fmad=false",
-         "-Xcompiler", "-fPIC,-O2", "-I", os.path.join(ROOT, "include"), "-I", CSRC]
+         "-Xcompiler", "-fPIC,-O2,-ffp-contract=off", "-I", os.path.join(ROOT, "include"), "-I", CSRC]
     if verbose:
         f += ["-Xptxas", "-v"]
     return f
