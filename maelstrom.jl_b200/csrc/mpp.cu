@@ -154,7 +154,7 @@ struct mpp_ctx {
     int cmg_ls, cmg_cs, cmg_tries;
     size_t cmg_smem;
     ClLev cmg_lev[CL_MAXLEV + 1];
-    int cmg_nd, cmg_nact;  // levels spread over the cluster, CTAs that hold planes of them
+    int cmg_nd, cmg_nact;  // 1: the first of them is spread over the cluster; CTAs that hold planes of it
     ClLists cmg_l;
     unsigned cmg_orb, cmg_ogi;
     // TMA tensor maps of the row-split levels the smoother streams with cp.async.bulk.tensor
@@ -1598,7 +1598,7 @@ int build_cmg(mpp_ctx* c) {
     const char* env = getenv("MPP_CMG");
     if ((env && !strcmp(env, "0")) || c->lb < 2) return MPP_OK;
     int64_t maxcells = CL_CELLS;
-    if (const char* mc = getenv("MPP_CMG_MAXCELLS")) maxcells = atoll(mc);
+    if (const char* mc = getenv("MPP_CMG_MAXCELLS")) maxcells = std::min<int64_t>(CL_CELLS, atoll(mc));
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->dev));
     const size_t cb = c->prec == MPP_PREC_FP64 ? 8 : 4;  // the arithmetic type
@@ -1611,9 +1611,10 @@ int build_cmg(mpp_ctx* c) {
         for (int ls = 1; ls < c->lb; ls++) {
             const int nl = c->L - 1 - ls;
             if (nl > CL_MAXLEV || cells(ls) > maxcells) continue;
-            int nd = 0;
-            while (nd < nl && cells(ls + nd) > CL_LOCAL_CELLS) nd++;
-            if (nd == nl) continue;  // (the level above the coarsest has at most 8 x 1024 cells)
+            // the first level is spread when it is above CL_LOCAL_CELLS; the next has an eighth of its cells,
+            // so it is not (and the level above the coarsest has at most 8 x 1024)
+            static_assert(CL_CELLS <= 8 * CL_LOCAL_CELLS, "one level is spread at most");
+            const int nd = cells(ls) > CL_LOCAL_CELLS ? 1 : 0;
             for (int cs : {CL_SIZE, CL_SIZE / 2}) {
                 if (nd == 0) cs = 1;
                 ClLev lev[CL_MAXLEV + 1];
@@ -1626,15 +1627,15 @@ int build_cmg(mpp_ctx* c) {
                     off += (bytes + 15) / 16 * 16;
                     return o;
                 };
-                // the top level's planes a CTA: whole planes of every spread level's, down to one
-                const int unit = 1 << nd, n3 = c->lv[ls].n[2], P0 = unit * ((n3 / unit + cs - 1) / cs);
+                // the spread level's planes a CTA: whole planes of the next level
+                const int n3 = c->lv[ls].n[2], P0 = 2 * ((n3 / 2 + cs - 1) / cs);
                 for (int q = 0; q <= nl && ok; q++) {
                     const LevelBuf& b = c->lv[ls + q];
                     ClLev& S = lev[q];
                     S.n1 = b.n[0];
                     S.n2 = b.n[1];
                     S.n3 = b.n[2];
-                    S.P = q < nd ? P0 >> q : S.n3;
+                    S.P = q < nd ? P0 : S.n3;
                     S.RS = (S.n1 + 1) / 2 + 1;
                     S.PS = (S.n2 + 1) * S.RS;
                     S.CS = (S.P + 2) * S.PS + S.RS + 1;

@@ -3,7 +3,7 @@
 //
 // From about 32^3 cells down a pass of a level is far less work than a launch costs, and most of
 // a V-cycle's passes are on these levels. Here the levels ls .. L-1 run in one launch:
-//   * the levels above LOCAL_CELLS are spread over the cluster, CTA r holding planes
+//   * the first one, when it is above CL_LOCAL_CELLS, is spread over the cluster, CTA r holding planes
 //     [r P, r P + P) with one halo plane each side; after each pass a CTA pushes its boundary
 //     planes' new values into its neighbours' halos (st.async, whose bytes complete a
 //     transaction barrier there), and waits for theirs: the exchange is one one-way trip between
@@ -88,7 +88,7 @@ struct ClLists {
     int4* cnt;       // [level][CTA]: cells of each colour; of each colour that the neighbours push here
     uint4* rb;       // the coarsest's unknowns by colour, RB_HALF places each
     int* nrb;        // and their numbers
-    void* share;     // level nd's x as CTA 0 holds it
+    void* share;     // the level's x below the spread one, as CTA 0 holds it
 };
 template <class M>
 struct ClArgs {
@@ -96,7 +96,7 @@ struct ClArgs {
     ClLev s[CL_MAXLEV + 1];   // and the coarsest (x only)
     BotLev cl;                // the coarsest
     ClLists l;
-    int nl, nd, nact;         // levels above the coarsest; spread ones; CTAs that hold planes of those
+    int nl, nd, nact;         // levels above the coarsest; 1: the first is spread; CTAs that hold planes of it
     int sweeps, coarse;
     unsigned orb, ogi;        // byte offsets of the coarsest's unknowns and of the top level's global places
     int* fault;
@@ -168,9 +168,6 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_lists(const __grid_const
         const ClLev &S = a.s[q], &D = a.s[q + 1];
         const auto& G = a.g[q];
         const int kb = spread ? me * S.P : 0, left = S.n3 - kb, np = left < 0 ? 0 : (left < S.P ? left : S.P);
-        const int cb = q + 1 < a.nd ? me * D.P : 0;  // the coarse level's first plane held
-        const int fb = q >= 1 && q - 1 < a.nd ? me * a.s[q - 1].P : 0;  // the finer one's (entries of a level that is
-                                                                        // restricted into from its own CTA)
         const int n = np * S.n2 * S.n1, H = S.n1 >> 1;
         const int64_t g0 = (int64_t)kb * S.n1 * S.n2;
         const bool lo = spread && me > 0, hi = spread && me + 1 < a.nact;
@@ -195,8 +192,8 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_lists(const __grid_const
             w.x = (uint32_t)cl_place(S, kk + 1, j, i >> 1) | (ci ? CL_CI : 0u) | (cj ? CL_CJ : 0u) | (ck ? CL_CK : 0u) |
                   ((lo && kk == 0) ? CL_LO : 0u) | ((hi && kk + 1 == np) ? CL_HI : 0u) |
                   (((A + B + K + 1) & 1) ? CL_P0 : 0u) | ((A & 1) ? CL_DH : 0u) | ((uint32_t)d << CL_DG);
-            w.y = (uint32_t)cl_place(D, K - cb + 1, B, A >> 1);
-            if (q > 0) w.y |= (uint32_t)((2 * k - fb) * a.s[q - 1].PS + 2 * j * a.s[q - 1].RS + i + 1) << 16;
+            w.y = (uint32_t)cl_place(D, K + 1, B, A >> 1);
+            if (q > 0) w.y |= (uint32_t)(2 * k * a.s[q - 1].PS + 2 * j * a.s[q - 1].RS + i + 1) << 16;
 #pragma unroll
             for (int cc = 0; cc < 2; cc++) {
                 const unsigned m = __ballot_sync(0xffffffffu, on && c == cc);
@@ -523,7 +520,7 @@ struct ClRun {
         }
         return Pr::scaled ? s : (C)4 * s;
     }
-    // into level q + 1, held as level q is (both spread, or both in this CTA)
+    // into level q + 1, both in this CTA
     __device__ __forceinline__ void restrict_into() {
         const ClLev& S = a.s[q + 1];
         const int4 c = sh.cnt[q + 1];
@@ -536,7 +533,7 @@ struct ClRun {
         }
         __syncthreads();
     }
-    // into level q + 1 of CTA 0 from the spread level q: this CTA's share of its planes
+    // into the next level, in CTA 0, from the spread one: this CTA's share of its planes
     __device__ __forceinline__ void restrict_out(int planes) {
         const ClLev& S = a.s[q + 1];
         const auto& G = a.g[q + 1];
@@ -708,11 +705,11 @@ __device__ __forceinline__ void cluster_dev(const ClArgs<typename Pr::M>& a) {
     // down
 #pragma unroll 1
     for (int q = 0; q < a.nl; q++) {
-        if (spread && q == a.nd) cluster_barrier();  // level nd's right-hand side is in CTA 0
+        if (spread && q == 1) cluster_barrier();  // level 1's right-hand side is in CTA 0
         if (q < a.nd ? !holds : !first) continue;
         if (q > 0) r.enter(q);
         r.down();
-        if (q + 1 == a.nd) r.restrict_out(np >> q);
+        if (spread && q == 0) r.restrict_out(np);
         else if (q + 1 < a.nl) r.restrict_into();
     }
     // coarse_kernel! (src/flip.jl:935-962), the right-hand side restricted into registers
@@ -760,16 +757,16 @@ __device__ __forceinline__ void cluster_dev(const ClArgs<typename Pr::M>& a) {
     // up
 #pragma unroll 1
     for (int q = a.nl - 1; q >= 0; q--) {
-        if (spread && q == a.nd - 1) {
-            if (first) {  // level nd's x as it lies here, for the other CTAs
+        if (spread && q == 0) {
+            if (first) {  // level 1's x as it lies here, for the other CTAs
                 const uint4* x = reinterpret_cast<const uint4*>(r.X);
                 for (int u = tid; u < (int)((2 * r.CS * sizeof(C) + 15) / 16); u += CL_THREADS)
                     static_cast<uint4*>(a.l.share)[u] = x[u];
             }
             cluster_barrier();
-            if (holds && !first) {  // the planes that this CTA's cells of level nd - 1 read, at their places
-                const ClLev& D = a.s[a.nd];
-                const int k0 = (kb >> (a.nd - 1)) / 2, m = ((np >> (a.nd - 1)) / 2 + 2) * D.PS + D.RS;
+            if (holds && !first) {  // the planes that this CTA's cells read, at their places
+                const ClLev& D = a.s[1];
+                const int k0 = kb / 2, m = (np / 2 + 2) * D.PS + D.RS;
                 const C* x = static_cast<const C*>(a.l.share);
                 C* Y = cl_ptr<C>(D.ox);
                 for (int t = tid; t < 2 * m; t += CL_THREADS) {
