@@ -42,8 +42,9 @@
 // mix passes p and p + 2, and none of its values of pass p + 1 lands before this CTA has read what
 // they replace. (By bytes alone a CTA whose neighbours' facing planes are dry waits for nobody.)
 // The arrivals are on their way while the pass works, sent by threads of the last warps (thread 0
-// sending them before its cells: 64^3 1.8 % slower, 256^3 0.9 %). Bytes alone against this form, beside
-// the tree before k_cluster: 64^3 1.44x and 1.45x, 96^3 rollout 1.32x and 1.29x, 256^3 1.04x and 1.03x.
+// sending them before its cells: 64^3 1.8 % slower, 256^3 0.9 %). Projections, us, bytes alone and with
+// the arrivals: 64^3 1022-1027 and 1015, 256^3 FP16 1.04 and 1.03 times the speed of the tree before
+// k_cluster, the 96^3 rollout 1.32 and 1.30 times.
 //
 // Every thread of every CTA runs the same cluster barriers; waits on the exchange are bounded
 // (the fault flag is set; that CTA waits, arrives and pushes no more, so its neighbours' waits give

@@ -3,10 +3,10 @@
 // (P. Markstein, IBM J. Res. Dev. 34, 1990: a faithful estimate corrected so is the rounded quotient).
 // The result is the IEEE quotient bit for bit over the ranges stated, but for the sign of a zero; an
 // infinite or NaN quotient stays one of the two (an infinite a gives NaN), so no finite value differs.
-// Keeping infinities and -0 too (a select beside the chain) costs the launches that are chains of
-// these 1 %: 32^3 projection 510 -> 516 us, 64^3 1076 -> 1087, a small sparse basin 1360 -> 1377; a
-// branch as much as the division it avoids (a half-sweep of the coarsest solve at 128 threads 157 cycles,
-// with the division 144, so 105).
+// Keeping infinities and -0 too (a select beside the chain) costs what is a chain of these 0.5 to 1 %
+// (32^3 projection 510 -> 513 us, 64^3 1076 -> 1084, a small sparse basin 1360 -> 1374, the runs' own
+// difference taken off); a branch as much as the division it avoids (a half-sweep of the coarsest solve
+// at 128 threads 157 cycles, with the division 144, so 105).
 // (Plain C++ but for the qualifiers: tests/test_division.py checks these statements on the CPU.)
 #pragma once
 

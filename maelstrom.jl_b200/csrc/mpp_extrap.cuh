@@ -180,8 +180,11 @@ __global__ void __launch_bounds__(TPB) k_extrap_flags4(ExtBits E) {
 // word; the words on the front are gathered in shared memory and shared out over the block's warps, a
 // lane a face (so a row's values are consecutive loads), LAYER_WW words a warp at a time. A warp's
 // words follow each other, the next words are another block's: a front, which is a sheet of words that
-// follow each other, meets every SM. (A thread that took its word's 32 faces alone: 18 us a layer at
-// 256^3, here 15.) `from_a`: the layer reads ra and writes rb (else the other way round).
+// follow each other, meets every SM. One form for all sizes: a call of 6 layers on the device, us, at
+// 16 x 16 x 32, 32^3, 64^3, 128^3, 256^3: 20, 23, 26, 41, 182; a thread that takes its word's 32 faces
+// alone 33, 63, 64, 85, 204; a list a warp in place of the block's, without the barriers, 47, 67, 81, 96,
+// 237 (few warps hold most of a front). `from_a`: the layer reads ra and writes rb (else the other way
+// round).
 constexpr int LAYER_WW = 4;
 __global__ void __launch_bounds__(TPB) k_extrap_layer(ExtBits E, int from_a) {
     pdl_wait();

@@ -1,5 +1,5 @@
-"""The V-cycle's small levels run in one thread-block cluster (k_cmg: levels of 32^3 cells
-and fewer, resident in the cluster's shared memory) or as per-level launches
+"""The V-cycle's small levels run as one launch on one thread-block cluster (k_cluster: levels of
+65 536 cells and fewer, the coarsest included, in its shared memory) or as per-level launches
 (MPP_CMG=0). With the same one-CTA bottom bound (MPP_BOTTOM_CELLS=512 for both), every
 pass computes the same arithmetic in the same order, so a projection must agree bit for
 bit, iteration count included, in every precision form."""

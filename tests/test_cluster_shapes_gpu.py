@@ -1,6 +1,6 @@
 """k_cluster (the small levels in one launch) against the per-level launches and the one-CTA bottom
-solve, bit for bit, over the shapes at which its layout changes: levels in one CTA alone, one or two
-levels spread over the cluster, planes that do not divide by the cluster, an odd coarsest level, more
+solve, bit for bit, over the shapes at which its layout changes: levels in one CTA alone, one
+level spread over the cluster, planes that do not divide by the cluster, an odd coarsest level, more
 cells of a colour than a CTA's threads hold at once, and bottom levels above the coarsest."""
 import dataclasses
 import os
